@@ -38,6 +38,7 @@ EXTRA = {
     "cg.cu": ["--fmad=true"],
     "noalloc.cu": ["--fmad=true"],
     "cg1.cu": ["--fmad=true"],
+    "cg_res.cu": ["--fmad=true"],
 }
 
 

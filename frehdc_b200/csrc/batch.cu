@@ -11,7 +11,9 @@
 //     k_cg1_batch (FREHD_BATCH_CTA_GROUPS, the default): each domain solved by a group of
 //       CTAs whose size depends on the domain's own cell count only (multi-CTA
 //       groups on CTAs of their own; single-CTA domains, longest first, taken
-//       one after another by whichever CTA is free)
+//       one after another by whichever CTA is free).  Domains whose solver state
+//       fits on chip run in k_cgr_batch instead: each on as many CTAs as its tiles,
+//       the CTAs taking one domain after another in a fixed schedule
 //     k_cg1_tiles (FREHD_BATCH_TILE_LIST): the CG tiles of every domain form one
 //       list spread over all CTAs; each domain's sums are added in its own tile
 //       order, so its result depends neither on the mix nor on cells_per_cta
@@ -30,6 +32,7 @@
 
 #include "cg1.h"
 #include "cg_common.cuh"
+#include "cg_res.h"
 #include "domain_host.h"
 #include "frehd_internal.h"
 #include "kernels.cuh"
@@ -50,6 +53,9 @@ namespace {
 // one after another along a tile row: the domain's view is staged once for
 // them (frehd_batch_set_stencil_tiles; the default, and the largest allowed).
 constexpr int kTilesPerBlock = 4, kMaxTilesPerBlock = 8;
+// Time of a resident CG iteration without its cells' work, in units of one row per
+// thread (the schedule's cost model).
+constexpr double kResIterBase = 3.0;
 
 struct Slot {
   frehd_domain *d = nullptr;
@@ -102,7 +108,12 @@ struct frehd_batch {
   DevArray<CgJob> jobs;
   DevArray<CgJob> singles;  // single-CTA solves, longest first
   int nsingles = 0;
-  int any_mixed = 0;        // an admitted domain solves in mixed precision
+  int any_mixed = 0;        // one of these domains solves in mixed precision
+  // resident solves: every CTA's list, and the single-CTA ones
+  int capacity_res = 0;
+  DevArray<int> rstart;
+  DevArray<CgJob> rjobs, rsingles;
+  int nrsingles = 0, nrctas = 0, any_rmixed = 0;
   // tile-list packing
   int packing = FREHD_BATCH_CTA_GROUPS;
   int tiles_per_block = kTilesPerBlock;
@@ -135,6 +146,17 @@ int group_size(const frehd_batch *b, const frehd_domain *d) {
   long g = (long)std::ceil(cells / b->cells_per_cta);
   g = std::max(1L, std::min(g, std::min(ntiles, (long)b->capacity)));
   return (int)g;
+}
+
+// Rows per thread of domain d's resident solve in this batch (0: it streams).
+// cells_per_cta asks for tiles of that many cells (up to the largest tile): few
+// large tiles keep more domains in flight, many small ones shorten one solve.  By
+// the domain's size alone, so that its result is the same in any mix.
+int resident_rows(const frehd_batch *b, const frehd_domain *d) {
+  if (!d->res_rows) return 0;
+  for (int KR = d->res_rows; KR < kResMaxKR; KR *= 2)
+    if (kResTW * res_th(KR) >= b->cells_per_cta) return KR;
+  return kResMaxKR;
 }
 
 // CTAs the batch needs with the given domains: the multi-CTA groups plus one
@@ -183,10 +205,16 @@ int launch_step(frehd_batch *b) {
   const dim3 bb(32, 8);
   k_explicit_batch<<<(unsigned)b->ntiles, bb, 0, b->stream>>>(b->views2.p, b->tiles.p);
   const bool tl = b->packing == FREHD_BATCH_TILE_LIST;
-  int rc = tl ? cg1_launch_tiles(b->views2.p, b->maps.p, b->bdoms.p, b->bstates.p, b->btiles.p,
+  int rc = FREHD_OK;
+  if (!tl && b->nrctas > 0)
+    rc = cgr_launch_batch(b->views2.p, b->rstart.p, b->rjobs.p, b->rsingles.p, b->nrsingles,
+                          &b->bsync.p->taken, b->nrctas, b->any_rmixed, b->stream);
+  if (rc) return rc;
+  if (b->nctas > 0)
+    rc = tl ? cg1_launch_tiles(b->views2.p, b->maps.p, b->bdoms.p, b->bstates.p, b->btiles.p,
                                  b->nbdoms, b->nbtiles, b->bpartials.p, b->bsync.p, b->bpart.p,
                                  b->nctas, b->stream)
-              : cg1_launch_batch(b->views2.p, b->maps.p, b->job_start.p, b->jobs.p, b->singles.p,
+            : cg1_launch_batch(b->views2.p, b->maps.p, b->job_start.p, b->jobs.p, b->singles.p,
                                  b->nsingles, &b->bsync.p->n_done, b->nctas, b->any_mixed,
                                  b->stream);
   if (rc) return rc;
@@ -247,6 +275,7 @@ int rebuild(frehd_batch *b) {
   b->ntiles_upwind = 0;
   b->nfin = 0;
   b->nctas = 0;
+  b->nrctas = 0;
   if (doms.empty()) {
     b->dirty = false;
     return FREHD_OK;
@@ -270,10 +299,12 @@ int rebuild(frehd_batch *b) {
   // CTA-group packing: multi-CTA groups on CTAs of their own; single-CTA
   // domains in one list that every CTA takes from once its own jobs are done.
   std::vector<std::vector<CgJob>> per_cta;
-  std::vector<Dom> singles;
+  std::vector<Dom> singles, resident;
   for (const Dom &m : doms) {
     if (b->packing == FREHD_BATCH_TILE_LIST) break;
-    if (m.g > 1) {
+    if (resident_rows(b, b->slots[m.slot].d)) {
+      resident.push_back(m);
+    } else if (m.g > 1) {
       for (int r = 0; r < m.g; ++r) per_cta.push_back({CgJob{m.slot, r, m.g, flags_of(m.slot)}});
     } else {
       singles.push_back(m);
@@ -298,6 +329,38 @@ int rebuild(frehd_batch *b) {
     jobs.insert(jobs.end(), per_cta[c].begin(), per_cta[c].end());
   }
   start[per_cta.size()] = (int)jobs.size();
+  // resident solves, largest first: each takes the CTAs that are free the soonest
+  // (a group starts together, when the last of its CTAs is free); the single-CTA
+  // ones are handed out at the end
+  std::stable_sort(resident.begin(), resident.end(),
+                   [](const Dom &a, const Dom &c) { return a.cells > c.cells; });
+  std::vector<std::vector<CgJob>> rlists(b->capacity_res);
+  std::vector<double> busy(b->capacity_res, 0.0);
+  std::vector<int> by_load(b->capacity_res);
+  std::iota(by_load.begin(), by_load.end(), 0);
+  std::vector<CgJob> rsingle_jobs;
+  for (const Dom &m : resident) {
+    const frehd_domain *d = b->slots[m.slot].d;
+    const int rows = resident_rows(b, d), flags = flags_of(m.slot) | rows << 4;
+    const int nb = (int)res_tiles(d->gr.nx, d->gr.ny, rows);
+    if (nb == 1) {
+      rsingle_jobs.push_back(CgJob{m.slot, 0, 1, flags});
+      continue;
+    }
+    std::stable_sort(by_load.begin(), by_load.end(), [&](int a, int c) { return busy[a] < busy[c]; });
+    const double end = busy[by_load[nb - 1]] + kResIterBase + rows;
+    for (int r = 0; r < nb; ++r) {
+      rlists[by_load[r]].push_back(CgJob{m.slot, r, nb, flags});
+      busy[by_load[r]] = end;
+    }
+  }
+  std::vector<int> rstart(b->capacity_res + 1, 0);
+  std::vector<CgJob> rjobs;
+  for (int c = 0; c < b->capacity_res; ++c) {
+    rstart[c] = (int)rjobs.size();
+    rjobs.insert(rjobs.end(), rlists[c].begin(), rlists[c].end());
+  }
+  rstart[b->capacity_res] = (int)rjobs.size();
 
   int rc = 0;
   rc = rc ? rc : b->views2.reserve(views.size());
@@ -307,6 +370,9 @@ int rebuild(frehd_batch *b) {
   rc = rc ? rc : b->job_start.reserve(start.size());
   rc = rc ? rc : b->jobs.reserve(jobs.size());
   rc = rc ? rc : b->singles.reserve(single_jobs.size());
+  rc = rc ? rc : b->rstart.reserve(rstart.size());
+  rc = rc ? rc : b->rjobs.reserve(rjobs.size());
+  rc = rc ? rc : b->rsingles.reserve(rsingle_jobs.size());
   {  // the launch counter (both packings), zeroed once and reset by k_finish_batch
     const bool fresh_sync = b->bsync.cap == 0;
     rc = rc ? rc : b->bsync.reserve(1);
@@ -331,6 +397,12 @@ int rebuild(frehd_batch *b) {
   if (!single_jobs.empty())
     BATCH_TRY(cudaMemcpyAsync(b->singles.p, single_jobs.data(), sizeof(CgJob) * single_jobs.size(),
                               cudaMemcpyHostToDevice, b->stream));
+  if (!resident.empty()) {
+    BATCH_TRY(cudaMemcpyAsync(b->rstart.p, rstart.data(), sizeof(int) * rstart.size(), cudaMemcpyHostToDevice, b->stream));
+    BATCH_TRY(cudaMemcpyAsync(b->rjobs.p, rjobs.data(), sizeof(CgJob) * rjobs.size(), cudaMemcpyHostToDevice, b->stream));
+    BATCH_TRY(cudaMemcpyAsync(b->rsingles.p, rsingle_jobs.data(), sizeof(CgJob) * rsingle_jobs.size(),
+                              cudaMemcpyHostToDevice, b->stream));
+  }
   if (tl) {
     BATCH_TRY(cudaMemcpyAsync(b->bdoms.p, bd.data(), sizeof(BDom) * bd.size(), cudaMemcpyHostToDevice, b->stream));
     BATCH_TRY(cudaMemcpyAsync(b->btiles.p, bt.data(), sizeof(BTile) * bt.size(), cudaMemcpyHostToDevice, b->stream));
@@ -342,8 +414,11 @@ int rebuild(frehd_batch *b) {
   b->nfin = (int)fins.size();
   b->nctas = tl ? b->capacity_tiles : (int)per_cta.size();
   b->nsingles = (int)single_jobs.size();
-  b->any_mixed = 0;
+  b->nrsingles = (int)rsingle_jobs.size();
+  b->nrctas = resident.empty() ? 0 : b->capacity_res;
+  b->any_mixed = b->any_rmixed = 0;
   for (const Dom &m : doms) b->any_mixed |= b->slots[m.slot].d->p.mixed ? 1 : 0;
+  for (const Dom &m : resident) b->any_rmixed |= b->slots[m.slot].d->p.mixed ? 1 : 0;
   b->nbdoms = (int)bd.size();
   b->nbtiles = (int)bt.size();
   b->dirty = false;
@@ -397,7 +472,8 @@ extern "C" int frehd_domain_footprint(const frehd_config *cfg, int r, long long 
   if (cfg->useScalar && cfg->nscalar > 1) b += 2 * 8 * tot * (long long)(cfg->nscalar - 1);  // tracers
   b += 36 * 8 * tot;                // persistent, per-step and CG arrays
   b += tot;                         // rmv flags
-  b += 4 * N + 2 * 8 * T;           // fix list, staging
+  b += 4 * N + 8 * T;               // fix list, staging
+  b += cgr_exchange_bytes(g, res_rows(cfg->nx, cfg->ny, 148));  // the resident solve's exchange
   b += 8 * std::max(nvel, 8LL * 148 + 8) + 4096;  // partials, scratch, maps
   b += 8 * N * (long long)r * r;    // fine bottoms
   b += (20 * 8 + 2 * 4) * tot;      // level-value cache of the fine geometry
@@ -417,6 +493,7 @@ extern "C" int frehd_batch_create(int device, long long hbm_budget_bytes, double
   b->cells_per_cta = cells_per_cta;
   int rc = cg1_batch_capacity(device, &b->capacity);
   if (!rc) rc = cg1_tiles_capacity(device, &b->capacity_tiles);
+  if (!rc) rc = cgr_capacity(device, &b->capacity_res);
   if (!rc && cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess)
     rc = fail(FREHD_ERR_CUDA, "stream creation failed");
   if (rc) {
@@ -447,6 +524,9 @@ extern "C" int frehd_batch_destroy(frehd_batch *b) {
   b->job_start.release();
   b->jobs.release();
   b->singles.release();
+  b->rstart.release();
+  b->rjobs.release();
+  b->rsingles.release();
   b->bdoms.release();
   b->btiles.release();
   b->bstates.release();
@@ -553,7 +633,7 @@ extern "C" int frehd_batch_info(frehd_batch *b, frehd_batch_info_t *out) {
   int n = 0;
   for (const Slot &s : b->slots) n += s.d != nullptr;
   out->domains = n;
-  out->cg_ctas = b->nctas;
+  out->cg_ctas = std::max(b->nctas, b->nrctas);
   out->cg_capacity = b->packing == FREHD_BATCH_TILE_LIST ? b->capacity_tiles : b->capacity;
   out->tiles = b->ntiles;
   out->graph = b->graph_live;

@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "cg1.h"
+#include "cg_res.h"
 #include "domain.cuh"
 #include "domain_host.h"
 #include "frehd_internal.h"
@@ -159,6 +160,7 @@ View make_view_at(const frehd_domain *d, int cur) {
   w.dXP = d->dXP; w.dYP = d->dYP;
   w.lvc = d->lvc;
   w.lvi = d->lvi;
+  w.xch = d->xch;
   w.sc = d->sc;
   return w;
 }
@@ -252,6 +254,9 @@ long long take_noconv(frehd_domain *d) {
 }
 
 int launch_cg(frehd_domain *d, const View &w) {
+  // a domain whose solver state fits on chip keeps it there
+  if (d->cg_schedule == FREHD_CG_SINGLE_SWEEP && d->res_rows)
+    return cgr_launch(w, d->res_rows, d->x0_mode, d->eliminate, d->stream);
   if (d->cg_schedule == FREHD_CG_SINGLE_SWEEP)
     return cg1_launch(w, d->cg1_maps_dev, d->cg1_blocks_n, d->x0_mode, d->eliminate, d->stream);
   View wv = w;
@@ -371,7 +376,6 @@ extern "C" int frehd_domain_create(const frehd_config *cfg, int device, frehd_do
   }
   if (!r) r |= dalloc(d, &d->fix_list, d->N);
   if (!r) r |= dalloc(d, &d->stage, d->T);
-  if (!r) r |= dalloc(d, &d->stage2, d->T);
   if (!r) r |= dalloc(d, &d->sc, 1);
   if (!r) r |= dalloc(d, &d->out, 1);
   // CG launch size: all blocks co-resident (cooperative launch), no more blocks
@@ -384,6 +388,9 @@ extern "C" int frehd_domain_create(const frehd_config *cfg, int device, frehd_do
     long cap = (long)nsm * std::max(per, 1);
     d->cg_blocks = (int)std::max(1L, std::min(want, cap));
     r |= cg1_blocks(device, d->gr, &d->cg1_blocks_n);
+    if (!r) r |= cgr_capacity(device, &d->res_ctas);
+    if (!r && (d->res_rows = res_rows(d->gr.nx, d->gr.ny, d->res_ctas)) != 0)
+      r |= dalloc(d, &d->xch, (long)(cgr_exchange_bytes(d->gr, d->res_rows) / sizeof(uint4)));
   }
   if (!r) {
     const long nvel = (long)((d->gr.nx + 31) / 32) * ((d->gr.ny + 7) / 8);
@@ -739,12 +746,14 @@ extern "C" int frehd_domain_download_state(frehd_domain *d, frehd_state *st) {
   }
   if (st->uuYP || st->vvXP) {
     View w = make_view(d);
-    k_interp_velocity<<<(unsigned)((N + 255) / 256), 256, 0, d->stream>>>(w, d->stage, d->stage2);
-    CUDA_TRY(cudaGetLastError());
-    if (st->uuYP)
-      CUDA_TRY(cudaMemcpyAsync(st->uuYP, d->stage, sizeof(double) * N, cudaMemcpyDeviceToHost, d->stream));
-    if (st->vvXP)
-      CUDA_TRY(cudaMemcpyAsync(st->vvXP, d->stage2, sizeof(double) * N, cudaMemcpyDeviceToHost, d->stream));
+    double *h[2] = {st->uuYP, st->vvXP};
+    for (int a = 0; a < 2; ++a) {
+      if (!h[a]) continue;
+      k_interp_velocity<<<(unsigned)((N + 255) / 256), 256, 0, d->stream>>>(w, a ? nullptr : d->stage,
+                                                                            a ? d->stage : nullptr);
+      CUDA_TRY(cudaGetLastError());
+      CUDA_TRY(cudaMemcpyAsync(h[a], d->stage, sizeof(double) * N, cudaMemcpyDeviceToHost, d->stream));
+    }
   }
   CUDA_TRY(cudaStreamSynchronize(d->stream));
   return FREHD_OK;

@@ -96,6 +96,8 @@ struct Scratch {
   long long cg_noconv_steps; // running count of completed steps whose solve stopped at maxIter
   unsigned long long wait_limit_ns;  // bound of the grid-barrier waits (0: kBarrierTimeoutNs)
   int n_done;                // batched solve over a tile list: domains whose solve ended
+  int taken;                 // batched resident solve: single-CTA solves handed out
+  unsigned res_tag;          // resident solve: the last tag its exchange entries carry
   int pad2;
 };
 
@@ -138,6 +140,7 @@ struct View {
   // -1 = none) are padded grids like every cell array.
   double *lvc;
   int *lvi;
+  uint4 *xch;  // exchange entries of the resident solve (null: the domain does not fit it)
   Scratch *sc;
 };
 

@@ -51,7 +51,6 @@ struct frehd_domain {
   frehd::StepOut *out = nullptr;
   frehd::StepOut *out_host = nullptr;  // pinned
   double *stage = nullptr;      // device staging, T doubles
-  double *stage2 = nullptr;
   int cur = 0;
   int x0_mode = FREHD_X0_ZERO;
   int cg_blocks = 1;
@@ -60,6 +59,9 @@ struct frehd_domain {
   frehd::Cg1Maps cg1_maps{};
   frehd::Cg1Maps *cg1_maps_dev = nullptr;  // device copy read by the kernel
   int cg1_blocks_n = 1;
+  int res_ctas = 0;              // CTAs the resident solve may use on this device
+  int res_rows = 0;              // its rows per thread (0: the domain does not fit it)
+  uint4 *xch = nullptr;          // its exchange entries
   int geom_set = 0, ready = 0;
   frehd_step_stats last{};
   std::vector<void *> allocs;

@@ -1223,6 +1223,7 @@ __global__ void k_finish_batch(const View *views2, const FinishJob *jobs, Scratc
   if (bsync && blockIdx.x == 0 && threadIdx.x == 0) {
     bsync->bar_count = 0;
     bsync->n_done = 0;
+    bsync->taken = 0;
     bsync->status = FREHD_OK;
   }
   stage_view(views2, f.d, &sv, &s_cur, threadIdx.x, blockDim.x);
@@ -1277,8 +1278,8 @@ __global__ void k_interp_velocity(View w, double *uuYP, double *vvXP) {
   const long N = (long)w.gr.nx * w.gr.ny;
   if (t >= N) return;
   const int i = (int)(t % w.gr.nx), j = (int)(t / w.gr.nx);
-  uuYP[t] = uuYP_at(w, i, j);
-  vvXP[t] = vvXP_at(w, i, j);
+  if (uuYP) uuYP[t] = uuYP_at(w, i, j);
+  if (vvXP) vvXP[t] = vvXP_at(w, i, j);
 }
 
 // Assembled system in the reference's terms (row-major Gn*, transposed z, x).
