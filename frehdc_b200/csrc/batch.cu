@@ -493,7 +493,8 @@ extern "C" int frehd_batch_create(int device, long long hbm_budget_bytes, double
   b->cells_per_cta = cells_per_cta;
   int rc = cg1_batch_capacity(device, &b->capacity);
   if (!rc) rc = cg1_tiles_capacity(device, &b->capacity_tiles);
-  if (!rc) rc = cgr_capacity(device, &b->capacity_res);
+  int clustered = 0;
+  if (!rc) rc = cgr_capacity(device, &b->capacity_res, &clustered);
   if (!rc && cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess)
     rc = fail(FREHD_ERR_CUDA, "stream creation failed");
   if (rc) {

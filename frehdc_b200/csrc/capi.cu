@@ -256,7 +256,7 @@ long long take_noconv(frehd_domain *d) {
 int launch_cg(frehd_domain *d, const View &w) {
   // a domain whose solver state fits on chip keeps it there
   if (d->cg_schedule == FREHD_CG_SINGLE_SWEEP && d->res_rows)
-    return cgr_launch(w, d->res_rows, d->x0_mode, d->eliminate, d->stream);
+    return cgr_launch(w, d->res_rows, d->res_clustered, d->x0_mode, d->eliminate, d->stream);
   if (d->cg_schedule == FREHD_CG_SINGLE_SWEEP)
     return cg1_launch(w, d->cg1_maps_dev, d->cg1_blocks_n, d->x0_mode, d->eliminate, d->stream);
   View wv = w;
@@ -388,7 +388,7 @@ extern "C" int frehd_domain_create(const frehd_config *cfg, int device, frehd_do
     long cap = (long)nsm * std::max(per, 1);
     d->cg_blocks = (int)std::max(1L, std::min(want, cap));
     r |= cg1_blocks(device, d->gr, &d->cg1_blocks_n);
-    if (!r) r |= cgr_capacity(device, &d->res_ctas);
+    if (!r) r |= cgr_capacity(device, &d->res_ctas, &d->res_clustered);
     if (!r && (d->res_rows = res_rows(d->gr.nx, d->gr.ny, d->res_ctas)) != 0)
       r |= dalloc(d, &d->xch, (long)(cgr_exchange_bytes(d->gr, d->res_rows) / sizeof(uint4)));
   }

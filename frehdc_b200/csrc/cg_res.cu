@@ -1,6 +1,10 @@
 // Kernels of the resident solve (cg_res.cuh): one domain, or many in a batch.
 #include "cg_res.cuh"
 
+#include <map>
+#include <mutex>
+#include <vector>
+
 #include "frehd_internal.h"
 
 namespace frehd {
@@ -25,42 +29,89 @@ __device__ __forceinline__ void sys_of(const View &w, int x0_surface, int elimin
   s->xbuf = w.xch;
 }
 
-// The domain's solve in its configured precision by nb CTAs.
-template <int KR, bool kMix>
-__device__ __forceinline__ bool res_solve(const ResSys &s, int mixed, double eps_inner, unsigned rank, unsigned nb,
-                                          double *sm, ResShared *sh) {
-  if (test_skip_barrier(s.sc, rank)) {  // a lone CTA has no partner whose wait could run out
-    if (nb == 1 && threadIdx.x == 0) set_status(s.sc, FREHD_ERR_TIMEOUT);
-    return false;
+// The two solves as functions of their own: in one kernel with each other or with
+// other tile heights they must not share a register allocation (the inlined FP32
+// sweeps of 64 x 64 tiles spilled 2.6 KB).
+template <int KR>
+__device__ __noinline__ int res_job_mixed(const ResSys *sp, double eps_inner, unsigned rank, unsigned nb,
+                                          unsigned csize) {
+  extern __shared__ __align__(16) double res_sm[];
+  __shared__ ResShared sh;
+  const ResSys s = *sp;
+  return res_mixed<KR>(s, eps_inner, rank, nb, csize, res_sm, &sh);
+}
+template <int KR>
+__device__ __noinline__ bool res_job_fp64(const ResSys *sp, unsigned rank, unsigned nb, unsigned csize) {
+  extern __shared__ __align__(16) double res_sm[];
+  __shared__ ResShared sh;
+  const ResSys s = *sp;
+  return res_fp64<KR>(s, rank, nb, csize, res_sm, &sh);
+}
+
+// The domain's solve in its configured precision by nb CTAs (in clusters of csize); sp
+// in shared memory.  kAlone: the FP64 solve is the kernel's only one (inlined: 4.56 us
+// per iteration at 512 x 512 against 5.39).
+template <int KR, bool kMix, bool kAlone = false>
+__device__ __forceinline__ void res_solve(const ResSys *sp, int mixed, double eps_inner, unsigned rank, unsigned nb,
+                                          unsigned csize) {
+  if (test_skip_barrier(sp->sc, rank)) {  // a lone CTA has no partner whose wait could run out
+    if (nb == 1 && threadIdx.x == 0) set_status(sp->sc, FREHD_ERR_TIMEOUT);
+    return;
   }
   if (kMix && mixed) {
-    const int r = res_mixed<KR>(s, eps_inner, rank, nb, sm, sh);
-    if (r != 2) return r == 1;
-    const bool ok = res_fp64<KR>(s, rank, nb, sm, sh);
-    if (ok && rank == 0 && threadIdx.x == 0) s.sc->cg_fallback = 2;
-    return ok;
+    if (res_job_mixed<KR>(sp, eps_inner, rank, nb, csize) != 2) return;
+    if (res_job_fp64<KR>(sp, rank, nb, csize) && rank == 0 && threadIdx.x == 0) sp->sc->cg_fallback = 2;
+    return;
   }
-  return res_fp64<KR>(s, rank, nb, sm, sh);
+  if (kAlone) {
+    extern __shared__ __align__(16) double res_sm[];
+    __shared__ ResShared sh;
+    const ResSys s = *sp;
+    res_fp64<KR>(s, rank, nb, csize, res_sm, &sh);
+  } else {
+    res_job_fp64<KR>(sp, rank, nb, csize);
+  }
 }
 
 }  // namespace
 
-template <int KR, bool kMix>
-__global__ void __launch_bounds__(kCgThreads, 1) k_cgr(View w, int x0_surface, int eliminate) {
-  if (*(volatile int *)&w.sc->status != FREHD_OK) return;
+// nb CTAs solve; the grid is a multiple of the cluster size csize, and the CTAs past
+// nb only keep their clusters whole.  fill(&s): the system, by one thread.
+template <int KR, bool kMix, class F>
+__device__ __forceinline__ void res_kernel(Scratch *sc, int mixed, double eps_inner, int nb, int csize, F fill) {
   extern __shared__ __align__(16) double res_sm[];
-  __shared__ ResShared sh;
-  ResSys s;
-  sys_of(w, x0_surface, eliminate, &s);
-  res_solve<KR, kMix>(s, w.p.mixed, w.p.eps_inner, blockIdx.x, gridDim.x, res_sm, &sh);
+  __shared__ ResSys s;
+  if (csize > 1) {
+    // the inbox carries no tag before a neighbour may write to it
+    uint4 *in = reinterpret_cast<uint4 *>(res_sm + kResSums * kResThreads + 3 * res_arr(KR));
+    for (int e = threadIdx.x; e < res_inbox(KR); e += kResThreads) in[e] = make_uint4(0, 0, 0, 0);
+    res_cluster_sync();
+  }
+  // (a step that has failed is skipped, but no CTA leaves its cluster early)
+  if ((int)blockIdx.x < nb && *(volatile int *)&sc->status == FREHD_OK) {
+    if (threadIdx.x == 0) fill(&s);
+    __syncthreads();
+    res_solve<KR, kMix, !kMix>(&s, mixed, eps_inner, blockIdx.x, nb, csize);
+  }
+  // no store into this CTA's shared memory is on its way any more
+  if (csize > 1) res_cluster_sync();
+}
+
+template <int KR, bool kMix>
+__global__ void __launch_bounds__(kResThreads, 1) k_cgr(View w, int x0_surface, int eliminate, int nb, int csize) {
+  res_kernel<KR, kMix>(w.sc, w.p.mixed, w.p.eps_inner, nb, csize,
+                       [&](ResSys *s) { sys_of(w, x0_surface, eliminate, s); });
+}
+
+template <int KR>
+__global__ void __launch_bounds__(kResThreads, 1) k_cgr_sys(ResSys sys, int nb, int csize) {
+  res_kernel<KR, false>(sys.sc, 0, 0.0, nb, csize, [&](ResSys *s) { *s = sys; });
 }
 
 template <bool kMix>
-__global__ void __launch_bounds__(kCgThreads, 1)
+__global__ void __launch_bounds__(kResThreads, 1)
     k_cgr_batch(const View *__restrict__ views2, const int *__restrict__ job_start,
                 const CgJob *__restrict__ jobs, const CgJob *__restrict__ singles, int nsingles, int *taken) {
-  extern __shared__ __align__(16) double res_sm[];
-  __shared__ ResShared sh;
   __shared__ ResSys s_sys;
   __shared__ double s_eps;
   __shared__ int s_mixed, s_next, s_run;
@@ -89,9 +140,9 @@ __global__ void __launch_bounds__(kCgThreads, 1)
     if (!s_run) continue;
     // a solve that gave up has marked its own domain; the CTA goes on with the next
     switch (jb.flags >> 4) {
-      case 1: res_solve<1, kMix>(s_sys, s_mixed, s_eps, jb.rank, jb.nb, res_sm, &sh); break;
-      case 2: res_solve<2, kMix>(s_sys, s_mixed, s_eps, jb.rank, jb.nb, res_sm, &sh); break;
-      default: res_solve<4, kMix>(s_sys, s_mixed, s_eps, jb.rank, jb.nb, res_sm, &sh); break;
+      case 1: res_solve<1, kMix>(&s_sys, s_mixed, s_eps, jb.rank, jb.nb, 1); break;
+      case 2: res_solve<2, kMix>(&s_sys, s_mixed, s_eps, jb.rank, jb.nb, 1); break;
+      default: res_solve<4, kMix>(&s_sys, s_mixed, s_eps, jb.rank, jb.nb, 1); break;
     }
   }
 }
@@ -107,26 +158,76 @@ void *single_fn(int rows, bool mix) {
     default: return mix ? (void *)k_cgr<4, true> : (void *)k_cgr<4, false>;
   }
 }
+void *sys_fn(int rows) {
+  switch (rows) {
+    case 1: return (void *)k_cgr_sys<1>;
+    case 2: return (void *)k_cgr_sys<2>;
+    default: return (void *)k_cgr_sys<4>;
+  }
+}
 void *batch_fn(bool mix) { return mix ? (void *)k_cgr_batch<true> : (void *)k_cgr_batch<false>; }
 
 }  // namespace
 
-int cgr_capacity(int device, int *ctas) {
-  int nsm = 0, least = 1 << 30;
+namespace {
+
+// Clusters of `size` CTAs of kernel fn that the device holds at once (0: none).
+int max_clusters(void *fn, unsigned smem, int size) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = size;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(size);
+  cfg.blockDim = dim3(kResThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+
+}  // namespace
+
+int cgr_capacity(int device, int *ctas, int *clustered) {
+  // found once per device; domains may be created on several host threads
+  static std::mutex mu;
+  static std::map<int, std::pair<int, int>> known;
+  std::lock_guard<std::mutex> lk(mu);
+  if (const auto it = known.find(device); it != known.end()) {
+    *ctas = it->second.first;
+    *clustered = it->second.second;
+    return FREHD_OK;
+  }
+  int nsm = 0, least = 1 << 30, clustered_n = kResClustered;
   cudaError_t e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
-  auto one = [&](void *fn, unsigned smem) {
+  auto one = [&](void *fn, unsigned smem, bool in_clusters) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int per = 0;
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kCgThreads, smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kResThreads, smem);
     if (per < least) least = per;
+    if (!in_clusters || e != cudaSuccess) return;
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return;
+    // as many CTAs as every form of cluster below that count allows
+    int n = max_clusters(fn, smem, kResFlat) < 1 ? 0 : 4 * max_clusters(fn, smem, 4);
+    if (8 * max_clusters(fn, smem, 8) < kResEights) n = n < kResFlat ? n : kResFlat;
+    if (n < clustered_n) clustered_n = n;
   };
+  for (int rows = kResMinKR; rows <= kResMaxKR; rows *= 2) one(sys_fn(rows), res_smem(rows), true);
   for (int mix = 0; mix < 2; ++mix) {
-    for (int rows = 1; rows <= kResMaxKR; rows *= 2) one(single_fn(rows, mix), res_smem(rows));
-    one(batch_fn(mix), res_smem(kResMaxKR));
+    for (int rows = kResMinKR; rows <= kResMaxKR; rows *= 2) one(single_fn(rows, mix), res_smem(rows), true);
+    one(batch_fn(mix), res_smem(kResMaxKR), false);
   }
   if (e != cudaSuccess) return fail(FREHD_ERR_CUDA, "resident solve set-up: %s", cudaGetErrorString(e));
   if (least < 1) return fail(FREHD_ERR_CUDA, "the resident solve does not fit on an SM");
   *ctas = nsm;  // one CTA per SM: more would share the SM's latency, not hide it
+  *clustered = clustered_n;
+  known[device] = {*ctas, *clustered};
   return FREHD_OK;
 }
 
@@ -139,21 +240,50 @@ long long cgr_exchange_bytes(const Grid &g, int rows) {
   return 16LL * n;
 }
 
-int cgr_launch(const View &w, int rows, int x0_surface, int eliminate, cudaStream_t stream) {
-  View wv = w;
-  int x0 = x0_surface, el = eliminate;
-  void *args[] = {&wv, &x0, &el};
-  const long nb = res_tiles(w.gr.nx, w.gr.ny, rows);
-  cudaError_t e = cudaLaunchCooperativeKernel(single_fn(rows, w.p.mixed != 0), dim3((unsigned)nb), dim3(kCgThreads),
-                                              args, res_smem(rows), stream);
-  if (e != cudaSuccess) return fail(FREHD_ERR_CUDA, "k_cgr launch: %s", cudaGetErrorString(e));
+namespace {
+
+// Kernel fn on the nb tiles of a solve, cooperatively and, where that fits, in clusters
+// (args: pointers to the kernel's own arguments; nb and the cluster size follow them).
+int launch_solve(void *fn, std::vector<void *> args, int nx, int ny, int rows, int clustered, cudaStream_t stream) {
+  int nb = (int)res_tiles(nx, ny, rows), csize = nb <= kResFlat ? nb : res_group(nb);
+  if (nb > clustered) csize = 1;
+  args.push_back(&nb);
+  args.push_back(&csize);
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = csize;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)((nb + csize - 1) / csize * csize));
+  cfg.blockDim = dim3(kResThreads);
+  cfg.dynamicSmemBytes = res_smem(rows);
+  cfg.stream = stream;
+  cfg.attrs = at;
+  cfg.numAttrs = csize > 1 ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args.data());
+  if (e != cudaSuccess) return fail(FREHD_ERR_CUDA, "resident solve launch: %s", cudaGetErrorString(e));
   return FREHD_OK;
+}
+
+}  // namespace
+
+int cgr_launch(const View &w, int rows, int clustered, int x0_surface, int eliminate, cudaStream_t stream) {
+  View wv = w;
+  return launch_solve(single_fn(rows, w.p.mixed != 0), {&wv, &x0_surface, &eliminate}, w.gr.nx, w.gr.ny, rows,
+                      clustered, stream);
+}
+
+int cgr_launch_sys(const ResSys &s, int rows, int clustered, cudaStream_t stream) {
+  ResSys sv = s;
+  return launch_solve(sys_fn(rows), {&sv}, s.nx, s.ny, rows, clustered, stream);
 }
 
 int cgr_launch_batch(const View *views2, const int *job_start, const CgJob *jobs, const CgJob *singles,
                      int nsingles, int *taken, int nctas, int any_mixed, cudaStream_t stream) {
   void *args[] = {&views2, &job_start, &jobs, &singles, &nsingles, &taken};
-  cudaError_t e = cudaLaunchCooperativeKernel(batch_fn(any_mixed != 0), dim3(nctas), dim3(kCgThreads), args,
+  cudaError_t e = cudaLaunchCooperativeKernel(batch_fn(any_mixed != 0), dim3(nctas), dim3(kResThreads), args,
                                               res_smem(kResMaxKR), stream);
   if (e != cudaSuccess) return fail(FREHD_ERR_CUDA, "k_cgr_batch launch: %s", cudaGetErrorString(e));
   return FREHD_OK;

@@ -59,7 +59,8 @@ struct frehd_domain {
   frehd::Cg1Maps cg1_maps{};
   frehd::Cg1Maps *cg1_maps_dev = nullptr;  // device copy read by the kernel
   int cg1_blocks_n = 1;
-  int res_ctas = 0;              // CTAs the resident solve may use on this device
+  int res_ctas = 0;              // CTAs the resident solve may use on this device,
+  int res_clustered = 0;         // and how many of them in clusters
   int res_rows = 0;              // its rows per thread (0: the domain does not fit it)
   uint4 *xch = nullptr;          // its exchange entries
   int geom_set = 0, ready = 0;

@@ -16,15 +16,19 @@
 // synchronisation).  Two calls that overlap on the GPU (different streams, or
 // different host threads without ordering) use the same scratch and race.
 //
-// The kernel is the persistent Jacobi-PCG of cg.cu over caller-provided
-// row-major arrays (no ghost ring): identical tile decomposition, arithmetic
-// and fixed-order reductions.
+// A system that the resident solve (cg_res.cuh) can tile runs there, on the caller's
+// row-major arrays: a solve of 48 x 40 cells took 368 us through the persistent
+// kernel below, of 512 x 512 461 us, 13 us per iteration for two grid barriers.  The
+// kernel below, the persistent Jacobi-PCG of cg.cu without a ghost ring, is left for
+// the shapes that have more tiles than the device has SMs (a few columns wide and
+// many thousand rows high).
 #include <cuda_runtime.h>
 
 #include <cmath>
 #include <mutex>
 
 #include "cg_common.cuh"
+#include "cg_res.h"
 #include "frehd_internal.h"
 
 namespace {
@@ -50,8 +54,15 @@ struct NoAllocArgs {
   double *scratch;  // device address of g_noalloc_scratch (from cudaGetSymbolAddress)
 };
 
-__global__ void k_noalloc_reset(double *scratch) {
+// The counters that must start at zero, and the resident solve's exchange entries
+// (n of them): any solve before may have left numbers there.
+__global__ void k_noalloc_reset(double *scratch, long n) {
+  uint4 *e = reinterpret_cast<uint4 *>(scratch + kHeaderDoubles + kPartialDoubles);
+  for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x)
+    e[q] = make_uint4(0, 0, 0, 0);
+  if (blockIdx.x || threadIdx.x) return;
   Scratch *sc = reinterpret_cast<Scratch *>(scratch);
+  sc->res_tag = 0;
   sc->bar_count = 0;
   sc->status = FREHD_OK;
   sc->cg_iters = 0;
@@ -224,6 +235,7 @@ struct DeviceSetup {
   bool done = false;
   double *scratch = nullptr;
   int max_blocks = 0;
+  int res_ctas = 0, res_clustered = 0;  // the resident solve's capacity
 };
 constexpr int kMaxDevices = 64;
 DeviceSetup g_setup[kMaxDevices];
@@ -249,9 +261,24 @@ int setup_current_device(DeviceSetup **out) {
     s.scratch = static_cast<double *>(p);
     s.max_blocks = nsm * (per > 0 ? per : 1);
     if (s.max_blocks > kNoAllocMaxBlocks) s.max_blocks = kNoAllocMaxBlocks;
+    const int rc = cgr_capacity(dev, &s.res_ctas, &s.res_clustered);
+    if (rc) return rc;
     s.done = true;
   }
   *out = &s;
+  return FREHD_OK;
+}
+
+// The solve's iterations, residual and status, if the caller asks for them (waits).
+int read_result(const DeviceSetup *s, cudaStream_t st, int *iters, double *rel_residual) {
+  if (!iters && !rel_residual) return FREHD_OK;  // asynchronous: results land in x
+  Scratch h;
+  cudaError_t e = cudaMemcpyAsync(&h, s->scratch, sizeof(Scratch), cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) return fail(FREHD_ERR_CUDA, "reading the solve status: %s", cudaGetErrorString(e));
+  if (iters) *iters = h.cg_iters;
+  if (rel_residual) *rel_residual = h.cg_bb > 0 ? std::sqrt(h.cg_rr) / std::sqrt(h.cg_bb) : 0.0;
+  if (h.status != FREHD_OK) return fail(h.status, "frehd_cg_solve_noalloc: %s", frehd_status_string(h.status));
   return FREHD_OK;
 }
 
@@ -274,22 +301,25 @@ extern "C" int frehd_cg_solve_noalloc(int nx, int ny, const double *Ct, const do
   int rc = setup_current_device(&s);
   if (rc) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  k_noalloc_reset<<<1, 1, 0, st>>>(s->scratch);
+  const int rows = res_rows(nx, ny, s->res_ctas);
+  const long entries = rows ? res_entries(res_tiles(nx, ny, rows), rows) : 0;
+  if (2 * entries > 4 * kNoAllocMaxCells)
+    return fail(FREHD_ERR_INVALID, "frehd_cg_solve_noalloc: exchange buffer too small");
+  k_noalloc_reset<<<(unsigned)(entries / 1024 + 1), 256, 0, st>>>(s->scratch, entries);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(FREHD_ERR_CUDA, "reset launch: %s", cudaGetErrorString(e));
+  if (rows) {
+    ResSys sys{nx, ny, nx, 0, Ct, Gx, Gy, b, x0_from_x ? x : nullptr, x, eps, max_iter, 1,
+               reinterpret_cast<Scratch *>(s->scratch),
+               reinterpret_cast<uint4 *>(s->scratch + kHeaderDoubles + kPartialDoubles)};
+    if ((rc = cgr_launch_sys(sys, rows, s->res_clustered, st)) != FREHD_OK) return rc;
+    return read_result(s, st, iters, rel_residual);
+  }
   const long ntiles = (long)((nx + CTX - 1) / CTX) * ((ny + CTY - 1) / CTY);
   const int grid = (int)(ntiles < s->max_blocks ? ntiles : s->max_blocks);
   NoAllocArgs a{nx, ny, Ct, Gx, Gy, b, x, eps, max_iter, x0_from_x, s->scratch};
   void *args[] = {&a};
   e = cudaLaunchCooperativeKernel((void *)k_cg_noalloc, dim3(grid), dim3(kCgThreads), args, 0, st);
   if (e != cudaSuccess) return fail(FREHD_ERR_CUDA, "cooperative launch: %s", cudaGetErrorString(e));
-  if (!iters && !rel_residual) return FREHD_OK;  // asynchronous: results land in x
-  Scratch h;
-  e = cudaMemcpyAsync(&h, s->scratch, sizeof(Scratch), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) return fail(FREHD_ERR_CUDA, "reading the solve status: %s", cudaGetErrorString(e));
-  if (iters) *iters = h.cg_iters;
-  if (rel_residual) *rel_residual = h.cg_bb > 0 ? std::sqrt(h.cg_rr) / std::sqrt(h.cg_bb) : 0.0;
-  if (h.status != FREHD_OK) return fail(h.status, "frehd_cg_solve_noalloc: %s", frehd_status_string(h.status));
-  return FREHD_OK;
+  return read_result(s, st, iters, rel_residual);
 }
