@@ -224,7 +224,7 @@ int launch_step(frehd_batch *b) {
   if (b->ntiles > b->ntiles_upwind)
     k_update_vel_tvd_batch<<<(unsigned)(b->ntiles - b->ntiles_upwind), bb, 0, b->stream>>>(
         b->views2.p, b->tiles.p + b->ntiles_upwind);
-  k_finish_batch<<<(unsigned)b->nfin, 256, 0, b->stream>>>(b->views2.p, b->fins.p, b->bsync.p);
+  k_finish_batch<<<(unsigned)b->nfin, kFinishThreads, 0, b->stream>>>(b->views2.p, b->fins.p, b->bsync.p);
   BATCH_TRY(cudaGetLastError());
   return FREHD_OK;
 }

@@ -293,7 +293,7 @@ int launch_update(frehd_domain *d, const View &w, cudaEvent_t *ev = nullptr) {
   else
     k_update_vel<<<gb, bb, 0, d->stream>>>(w);
   mark(ev, 4, d->stream);
-  k_finish<<<1, 256, 0, d->stream>>>(w, (int)(gb.x * gb.y), d->out);
+  k_finish<<<1, kFinishThreads, 0, d->stream>>>(w, (int)(gb.x * gb.y), d->out);
   mark(ev, 5, d->stream);
   CUDA_TRY(cudaGetLastError());
   return FREHD_OK;
