@@ -185,8 +185,10 @@ __device__ __forceinline__ bool sweep(const SweepMaps &m, T *rn_out, T *pn_out, 
                                       const Grid &g, const TileIt &ti, unsigned rank, unsigned nb,
                                       T alpha, T beta, double (&red)[6], unsigned char *smem,
                                       unsigned long long *bars, unsigned &seq, Scratch *sc,
-                                      bool x_zero = false) {
+                                      bool flip, bool x_zero = false) {
   // x_zero: X starts from zero (its stored values are not read)
+  // flip: the tiles in reverse, so that every other sweep starts on what the last one
+  // left in L2
   using B = Box<T, TH>;
   constexpr int RW = B::kRowsPerWarp, NW = kCgThreads / 32;
   __shared__ int s_ok;
@@ -195,13 +197,14 @@ __device__ __forceinline__ bool sweep(const SweepMaps &m, T *rn_out, T *pn_out, 
   if (threadIdx.x == 0) {
     asm volatile("fence.proxy.async.global;" ::: "memory");
     if ((int)rank < ti.ntiles)
-      issue_tile<T, TH>(m, ti, rank, smem + (seq & 1) * B::kStageBytes, &bars[seq & 1]);
+      issue_tile<T, TH>(m, ti, flip ? ti.ntiles - 1 - (int)rank : rank, smem + (seq & 1) * B::kStageBytes,
+                        &bars[seq & 1]);
   }
-  for (int tile = rank; tile < ti.ntiles; tile += nb, ++seq) {
+  for (int at = rank; at < ti.ntiles; at += nb, ++seq) {
     const int st = seq & 1;
-    const int next = tile + (int)nb;
+    const int tile = flip ? ti.ntiles - 1 - at : at, next = at + (int)nb;
     if (threadIdx.x == 0 && next < ti.ntiles)
-      issue_tile<T, TH>(m, ti, next, smem + (st ^ 1) * B::kStageBytes, &bars[st ^ 1]);
+      issue_tile<T, TH>(m, ti, flip ? ti.ntiles - 1 - next : next, smem + (st ^ 1) * B::kStageBytes, &bars[st ^ 1]);
     int i0, j0;
     B::origin(ti, tile, &i0, &j0);
     // X and |Ct| of the owned cells: in flight while the boxes arrive
@@ -491,7 +494,7 @@ static __device__ __forceinline__ bool cg1_fp64(const View &w, const Cg1Maps *__
       double red[6] = {0, 0, 0, 0, 0, 0};
       const SweepMaps sm{&m->r[cur], &m->p[cur], &m->hx, &m->hy};
       if (!sweep<double, true, double>(sm, rn_out, pn_out, X, Ct, g, ti, rank, nb, alpha, beta, red,
-                                       smem, bars, seq, sc))
+                                       smem, bars, seq, sc, cur != 0))
         return false;
       if (!grid_allreduce<6, kRedStride>(red, sc, partials, totals, nb, rank)) return false;
       gamma_old = gamma;
@@ -696,7 +699,7 @@ static __device__ __forceinline__ int cg1_mixed(const View &w, const Cg1Maps *__
       // d~ starts from zero at the inner solve's first sweep
       if (!sweep<float, false, float, kTallTH>(sm, rn_out, pn_out, FD, Ct, g, ti2, rank, nb,
                                                (float)alpha, (float)beta, red, smem, bars, seq, sc,
-                                               it == 1))
+                                               cur != 0, it == 1))
         return 0;
       if (!grid_allreduce<6, kRedStride>(red, sc, partials, totals, nb, rank)) return 0;
       gamma_old = gamma;
