@@ -202,8 +202,8 @@ void drop_graph(frehd_batch *b) {
 }
 
 int launch_step(frehd_batch *b) {
-  const dim3 bb(32, 8);
-  k_explicit_batch<<<(unsigned)b->ntiles, bb, 0, b->stream>>>(b->views2.p, b->tiles.p);
+  const dim3 bb(32, 8), bh(32, 8 + kStencilHaloRows);
+  k_explicit_batch<<<(unsigned)b->ntiles, bh, 0, b->stream>>>(b->views2.p, b->tiles.p);
   const bool tl = b->packing == FREHD_BATCH_TILE_LIST;
   int rc = FREHD_OK;
   if (!tl && b->nrctas > 0)
@@ -218,7 +218,7 @@ int launch_step(frehd_batch *b) {
                                  b->nsingles, &b->bsync.p->n_done, b->nctas, b->any_mixed,
                                  b->stream);
   if (rc) return rc;
-  k_update_geo_batch<<<(unsigned)b->ntiles, bb, 0, b->stream>>>(b->views2.p, b->tiles.p);
+  k_update_geo_batch<<<(unsigned)b->ntiles, bh, 0, b->stream>>>(b->views2.p, b->tiles.p);
   if (b->ntiles_upwind > 0)
     k_update_vel_batch<<<(unsigned)b->ntiles_upwind, bb, 0, b->stream>>>(b->views2.p, b->tiles.p);
   if (b->ntiles > b->ntiles_upwind)

@@ -286,7 +286,7 @@ void mark(cudaEvent_t *ev, int slot, cudaStream_t st) {
 int launch_update(frehd_domain *d, const View &w, cudaEvent_t *ev = nullptr) {
   const dim3 gb = tile_grid(d), bb(32, 8);
   mark(ev, 2, d->stream);
-  k_update_geo<<<gb, bb, 0, d->stream>>>(w);
+  k_update_geo<<<gb, dim3(32, 8 + kStencilHaloRows), 0, d->stream>>>(w);
   mark(ev, 3, d->stream);
   if (d->p.scalarAdv == 2)
     k_update_vel_tvd<<<gb, bb, 0, d->stream>>>(w);
@@ -926,7 +926,7 @@ extern "C" int frehd_domain_init(frehd_domain *d, const double *bottom, const do
   if (rc) return rc;
   {
     View w = make_view(d);
-    k_update_geo_init<<<tile_grid(d), dim3(32, 8), 0, d->stream>>>(w);
+    k_update_geo_init<<<tile_grid(d), dim3(32, 8 + kStencilHaloRows), 0, d->stream>>>(w);
     CUDA_TRY(cudaGetLastError());
     std::swap(d->ind[0], d->ind[1]);  // the evaluated indices become current
   }
@@ -950,7 +950,7 @@ extern "C" int frehd_domain_phase(frehd_domain *d, int phase, int tt, const doub
   View w = make_view(d);
   if (phase == FREHD_PHASE_EXPLICIT) {
     k_set_tt<<<1, 1, 0, d->stream>>>(d->sc, tt);
-    k_explicit<<<tile_grid(d), dim3(32, 8), 0, d->stream>>>(w);
+    k_explicit<<<tile_grid(d), dim3(32, 8 + kStencilHaloRows), 0, d->stream>>>(w);
     CUDA_TRY(cudaGetLastError());
   } else if (phase == FREHD_PHASE_SOLVE) {
     int rc = launch_cg(d, w);
@@ -987,7 +987,7 @@ extern "C" int frehd_domain_run(frehd_domain *d, int t0, int nsteps) {
     View w = make_view(d);
     cudaEvent_t *ev = step_events(d, s);
     mark(ev, 0, d->stream);
-    k_explicit<<<tile_grid(d), dim3(32, 8), 0, d->stream>>>(w);
+    k_explicit<<<tile_grid(d), dim3(32, 8 + kStencilHaloRows), 0, d->stream>>>(w);
     mark(ev, 1, d->stream);
     int rc = launch_cg(d, w);
     if (rc) return rc;

@@ -28,6 +28,9 @@ __device__ __forceinline__ double warp_max(double v) {
   return v;
 }
 
+// rows of threads that k_explicit and k_update_geo (with their batched and initial
+// forms) have besides the tile's 32 x 8
+constexpr int kStencilHaloRows = 2;
 __global__ void k_explicit(View w);
 __global__ void k_update_geo(View w);
 __global__ void k_update_geo_init(View w);

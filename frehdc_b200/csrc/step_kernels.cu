@@ -26,6 +26,11 @@ namespace frehd {
 // ---------------------------------------------------------------- helpers
 // Thread-block tile of the stencil kernels: 32 cells along x (one warp) by 8 rows.
 constexpr int TBX = 32, TBY = 8, EX = TBX + 1, EY = TBY + 1;
+// k_explicit and k_update_geo evaluate a halo row and a halo column too, in two warps
+// of their own: done by the tile's first warps after their own cells they doubled the
+// block's chain of dependent loads.
+constexpr int THALO = kStencilHaloRows;
+static_assert(THALO == 2 && TBY <= TBX, "one warp for the halo row, one for the column");
 
 __device__ __forceinline__ double rd(const double *a, const Grid &g, int i, int j) {
   return a[g.at(i, j)];
@@ -189,38 +194,32 @@ __device__ __forceinline__ double gface(double coef, double N, double Vf, double
 // Writes EnXP/EnYP, the face coefficients Gx (east face) and Gy (north face),
 // the row diagonal Ct (negated for rows the reference decouples: tidal rows and
 // closed dry cells) and the right-hand side b, all in the padded layout.
-// A 32 x 8 block evaluates the explicit term of every x face and y face it
-// needs once: each thread its own east and north face, threads 0-31 the south
-// halo row's north faces and threads 32-39 the west halo column's east faces.
+// A block evaluates the explicit term of every x face and y face its 32 x 8 cells
+// need once: each thread its own east and north face, warp TBY the south halo row's
+// north faces and warp TBY + 1 the west halo column's east faces.
 static __device__ __forceinline__ void explicit_tile(const View &w, int bx, int by) {
   const Params &p = w.p;
   const Grid &g = w.gr;
   __shared__ double sEx[TBY][TBX + 1], sDx[TBY][TBX + 1];  // x faces, column 0 = west halo
   __shared__ double sEy[TBY + 1][TBX], sDy[TBY + 1][TBX];  // y faces, row 0 = south halo
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TBX + tx;
+  const int tx = threadIdx.x, ty = threadIdx.y;
   const int i0 = bx * TBX, j0 = by * TBY;
-  const int i = i0 + tx, j = j0 + ty;
-  const bool in = i < g.nx && j < g.ny;
+  // the cell whose x face and (or) y face this thread evaluates
+  const bool own = ty < TBY, south = ty == TBY;
+  const int i = own || south ? i0 + tx : i0 - 1;
+  const int j = own ? j0 + ty : (south ? j0 - 1 : j0 + tx);
+  const bool in = own && i < g.nx && j < g.ny;
   Ex ex{0.0, 0.0}, ey{0.0, 0.0};
-  if (in) {
-    ex = explicit_x(w, i, j);
-    ey = explicit_y(w, i, j);
+  // (ghosts never written: 0)
+  if (own ? in : !south && tx < TBY && i0 > 0 && j < g.ny) ex = explicit_x(w, i, j);
+  if (own ? in : south && i < g.nx && j0 > 0 && j < g.ny) ey = explicit_y(w, i, j);
+  if (own || (!south && tx < TBY)) {
+    sEx[own ? ty : tx][own ? tx + 1 : 0] = ex.En;
+    sDx[own ? ty : tx][own ? tx + 1 : 0] = ex.Drag;
   }
-  sEx[ty][tx + 1] = ex.En;
-  sDx[ty][tx + 1] = ex.Drag;
-  sEy[ty + 1][tx] = ey.En;
-  sDy[ty + 1][tx] = ey.Drag;
-  if (tid < TBX) {  // north faces of the row below the block (ghosts never written: 0)
-    Ex e{0.0, 0.0};
-    if (i0 + tid < g.nx && j0 > 0 && j0 - 1 < g.ny) e = explicit_y(w, i0 + tid, j0 - 1);
-    sEy[0][tid] = e.En;
-    sDy[0][tid] = e.Drag;
-  } else if (tid < TBX + TBY) {  // east faces of the column left of the block
-    const int t = tid - TBX;
-    Ex e{0.0, 0.0};
-    if (i0 > 0 && j0 + t < g.ny) e = explicit_x(w, i0 - 1, j0 + t);
-    sEx[t][0] = e.En;
-    sDx[t][0] = e.Drag;
+  if (own || south) {
+    sEy[own ? ty + 1 : 0][tx] = ey.En;
+    sDy[own ? ty + 1 : 0][tx] = ey.Drag;
   }
   __syncthreads();
   if (!in) return;
@@ -273,12 +272,11 @@ static __device__ __forceinline__ void explicit_tile(const View &w, int bx, int 
   w.b[k] = b;
 }
 
-// Six blocks per SM (40 registers, a few spills): the explicit terms wait on
-// their neighbour loads and IEEE divisions, and the extra warps hide them --
-// 1.58 ms per 4096^2 step against 1.83 at four blocks and 1.68 at five.
-constexpr int kExplicitMinBlocks = 6;
+// Five blocks per SM (40 registers, a few spills): the explicit terms wait on their
+// neighbour loads and IEEE divisions, and the extra warps hide them.
+constexpr int kExplicitMinBlocks = 5;
 
-__global__ void __launch_bounds__(TBX *TBY, kExplicitMinBlocks) k_explicit(View w) {
+__global__ void __launch_bounds__(TBX *(TBY + THALO), kExplicitMinBlocks) k_explicit(View w) {
   if (*(volatile int *)&w.sc->status != FREHD_OK) return;  // a fatal step stops the run
   explicit_tile(w, blockIdx.x, blockIdx.y);
 }
@@ -498,7 +496,7 @@ __device__ NewSurf new_surface(const View &w, int i, int j) {
 // four blocks pay for the spills: 1.85 ms per 4096^2 step against 2.01 at 3
 // and 2.27 at 2.
 #ifndef FREHD_GEO_MIN_BLOCKS
-#define FREHD_GEO_MIN_BLOCKS 4
+#define FREHD_GEO_MIN_BLOCKS 3
 #endif
 
 template <bool kInit>
@@ -509,24 +507,13 @@ static __device__ __forceinline__ void update_geo_tile(const View &w, int bx, in
   __shared__ double sh_Vxp[EY][EX], sh_Vxm[EY][EX], sh_Vyp[EY][EX], sh_Vym[EY][EX];
   __shared__ double sh_V[EY][EX], sh_Z[EY][EX];
   const int i0 = bx * TBX, j0 = by * TBY;
-  const int tid = threadIdx.y * TBX + threadIdx.x;
-  // Each thread evaluates its own cell; threads 0..TBX-1 then evaluate the north
-  // halo row (only Om, Vym, s are read from it) and threads TBX..TBX+TBY-1 the
-  // east halo column (only Nm, Vxm, s).
-  for (int pass = 0; pass < 2; ++pass) {
-    int ex, ey;
-    if (pass == 0) {
-      ex = threadIdx.x;
-      ey = threadIdx.y;
-    } else {
-      if (tid >= TBX + TBY) break;
-      ex = tid < TBX ? tid : TBX;
-      ey = tid < TBX ? TBY : tid - TBX;
-    }
+  // Each thread evaluates its own cell; warp TBY the north halo row (only Om, Vym, s are
+  // read from it) and warp TBY + 1 the east halo column (only Nm, Vxm, s).
+  const bool own = threadIdx.y < TBY, column = threadIdx.y > TBY;
+  const int ex = column ? TBX : threadIdx.x, ey = column ? threadIdx.x : threadIdx.y;
+  if (i0 + ex < g.nx && j0 + ey < g.ny && !(column && threadIdx.x >= TBY)) {
     const int i = i0 + ex, j = j0 + ey;
-    if (i >= g.nx || j >= g.ny) continue;
     const long k = g.at(i, j);
-    const bool own = pass == 0;
     double s;
     double depth_old = w.depth_cur[k];
     if (kInit) {
@@ -572,7 +559,7 @@ static __device__ __forceinline__ void update_geo_tile(const View &w, int bx, in
   __syncthreads();
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int i = i0 + tx, j = j0 + ty;
-  if (i >= g.nx || j >= g.ny) return;
+  if (ty >= TBY || i >= g.nx || j >= g.ny) return;
   // combineSubArea (subgrid.c:264-525), useminA = 0, useminV not 1/2, one rank
   const double dxdy = p.dx * p.dy;
   const double s = sh_s[ty][tx], Z = sh_Z[ty][tx];
@@ -648,13 +635,13 @@ static __device__ __forceinline__ void update_geo_tile(const View &w, int bx, in
   for (int a = 0; a < 8; ++a) arr[a][k] = val[a];
 }
 
-__global__ void __launch_bounds__(TBX *TBY, FREHD_GEO_MIN_BLOCKS) k_update_geo(View w) {
+__global__ void __launch_bounds__(TBX *(TBY + THALO), FREHD_GEO_MIN_BLOCKS) k_update_geo(View w) {
   if (*(volatile int *)&w.sc->status != FREHD_OK) return;
   update_geo_tile<false>(w, blockIdx.x, blockIdx.y);
 }
 
 // The geometry of the initial state (Init's computeSubArea + combineSubArea).
-__global__ void __launch_bounds__(TBX *TBY, FREHD_GEO_MIN_BLOCKS) k_update_geo_init(View w) {
+__global__ void __launch_bounds__(TBX *(TBY + THALO), FREHD_GEO_MIN_BLOCKS) k_update_geo_init(View w) {
   update_geo_tile<true>(w, blockIdx.x, blockIdx.y);
 }
 
@@ -1170,12 +1157,12 @@ static __device__ __forceinline__ void stage_view(const View *views2, int d, Vie
 // A block stages its domain's view once and runs the tile code on t.nt
 // consecutive tiles of one tile row (the barrier between them frees the
 // tile's shared memory for the next).
-__global__ void __launch_bounds__(TBX *TBY, kExplicitMinBlocks)
+__global__ void __launch_bounds__(TBX *(TBY + THALO), kExplicitMinBlocks)
     k_explicit_batch(const View *views2, const BatchTile *tiles) {
   __shared__ View sv;
   __shared__ int s_cur;
   const BatchTile t = tiles[blockIdx.x];
-  stage_view(views2, t.d, &sv, &s_cur, threadIdx.y * TBX + threadIdx.x, TBX * TBY);
+  stage_view(views2, t.d, &sv, &s_cur, threadIdx.y * TBX + threadIdx.x, TBX * (TBY + THALO));
   if (*(volatile int *)&sv.sc->status != FREHD_OK) return;
   for (int q = 0; q < t.nt; ++q) {
     if (q) __syncthreads();
@@ -1183,12 +1170,12 @@ __global__ void __launch_bounds__(TBX *TBY, kExplicitMinBlocks)
   }
 }
 
-__global__ void __launch_bounds__(TBX *TBY, FREHD_GEO_MIN_BLOCKS)
+__global__ void __launch_bounds__(TBX *(TBY + THALO), FREHD_GEO_MIN_BLOCKS)
     k_update_geo_batch(const View *views2, const BatchTile *tiles) {
   __shared__ View sv;
   __shared__ int s_cur;
   const BatchTile t = tiles[blockIdx.x];
-  stage_view(views2, t.d, &sv, &s_cur, threadIdx.y * TBX + threadIdx.x, TBX * TBY);
+  stage_view(views2, t.d, &sv, &s_cur, threadIdx.y * TBX + threadIdx.x, TBX * (TBY + THALO));
   if (*(volatile int *)&sv.sc->status != FREHD_OK) return;
   for (int q = 0; q < t.nt; ++q) {
     if (q) __syncthreads();  // also: the window's mbarrier is re-armed only after every wait on it
