@@ -272,8 +272,11 @@ static __device__ __forceinline__ void explicit_tile(const View &w, int bx, int 
   w.b[k] = b;
 }
 
-// Five blocks per SM (40 registers, a few spills): the explicit terms wait on their
-// neighbour loads and IEEE divisions, and the extra warps hide them.
+// Five blocks of 320 threads per SM (40 registers, a few spills): the explicit terms
+// wait on their neighbour loads and IEEE divisions, and the extra warps hide them:
+// 1.41 ms per 4096^2 step and 19 us at 128^2 (four blocks, 48 registers: 1.57 ms
+// and 17.8 us; six blocks of 256 threads with the halo on the first warps: 1.60 ms
+// and 23 us).
 constexpr int kExplicitMinBlocks = 5;
 
 __global__ void __launch_bounds__(TBX *(TBY + THALO), kExplicitMinBlocks) k_explicit(View w) {
@@ -490,11 +493,11 @@ __device__ NewSurf new_surface(const View &w, int i, int j) {
 // ---------------------------------------------------------------- k_update_geo
 // Shared-memory tile: each 32x8 block evaluates the subgrid half-cell values of
 // its cells plus one column east and one row north, then combines them.
-// Blocks of k_update_geo per SM the register allocation aims for (2: 128
-// registers without spills; 3: 80; 4: 64, with spill traffic to L1).  With the
-// level-value cache the kernel waits on dependent loads, so the extra warps of
-// four blocks pay for the spills: 1.85 ms per 4096^2 step against 2.01 at 3
-// and 2.27 at 2.
+// Blocks of k_update_geo per SM the register allocation aims for: with the
+// level-value cache the kernel waits on dependent loads, so warps in flight pay
+// for a few spills.  Three blocks of 320 threads (64 registers): 1.84 ms per 4096^2
+// step and 17 us at 128^2; four blocks of 256 threads, whose first warps do the
+// halo after their own cells (64 registers): 1.91 ms and 20 us.
 #ifndef FREHD_GEO_MIN_BLOCKS
 #define FREHD_GEO_MIN_BLOCKS 3
 #endif

@@ -412,7 +412,10 @@ int frehd_cg_solve_noalloc(int nx, int ny, const double *Ct, const double *Gx, c
  *   FREHD_BATCH_CTA_GROUPS (default): a domain's CG runs on
  *     ceil(cells / cells_per_cta) CTAs (at most its tile count) whatever the mix; the
  *     single-CTA solves, largest first, go to whichever CTA is free; admission
- *     also needs free CTAs;
+ *     also needs free CTAs.  A domain whose solver state fits on chip (up to about
+ *     600 K cells) runs instead on one CTA per tile of cells_per_cta cells (1024 to
+ *     4096), the CTAs taking such solves one after another; its admission counts
+ *     the same CTAs as before;
  *   FREHD_BATCH_TILE_LIST: every domain's CG tiles form one list spread over
  *     all CTAs; a domain's sums are added in its own tile order, so its result is
  *     the same in any mix; cells_per_cta is not used, and admission is by memory
