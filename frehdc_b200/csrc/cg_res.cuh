@@ -277,7 +277,7 @@ struct ResPair<float> {
 template <typename T, int KR>
 struct ResTile {
   T r[KR][2], p[KR][2], x[KR][2];
-  T hx[KR][3], hy[KR + 1][2];  // |couplings| of the rows' x faces (west, middle, east) and y faces
+  T hx[KR][3], hy[KR + 1][2];  // couplings of the rows' x faces (west, middle, east) and y faces
   T r1, h1[4], r2[2];          // ring cell; couplings east, west, north, south; outer and diagonal
   unsigned dec;                // bit 2k + c: decoupled cell; bit 31: decoupled ring cell
   int q1;                      // shared-memory position of the ring cell (-1: none)
@@ -375,7 +375,7 @@ __device__ __forceinline__ double res_residual_padded(const ResSys &s, const dou
   return __dsub_rn(bk, fma(ct, xk, -ax));
 }
 
-// The tile's couplings (scaled, |.|), decoupled flags and ring bookkeeping, by way
+// The tile's couplings (scaled), decoupled flags and ring bookkeeping, by way
 // of three shared arrays (loops over the tile and its rings: unrolled per thread,
 // the divisions alone were 30 KB of code that every solve fetched anew).
 template <typename T, int KR>
@@ -412,7 +412,7 @@ __device__ __forceinline__ void res_setup(const ResSys &s, const ResCtx &c, int 
       if (cy < TH + 3 && j + 1 < s.ny && !(elim && !(a > 0 && ds[e + kResPitch] > 0)))
         hy = s.Gy[k] / (fabs(a) * fabs(ds[e + kResPitch]));
     }
-    dx_[e] = fabs(hx);
+    dx_[e] = hx;
     dy_[e] = hy;
   }
   __syncthreads();

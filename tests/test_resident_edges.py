@@ -1,0 +1,51 @@
+"""The resident solve (csrc/cg_res.cuh) on systems that a time step does not assemble.
+
+Systems are diagonally dominant with smallest eigenvalue 1, as in
+test_resident_solve.py, whose bound on the true residual (the recursive one,
+1e-12 ||b||, and the recursion's rounding) holds for them too.
+"""
+import numpy as np
+import pytest
+
+from frehdc_b200 import native
+from tests.test_resident_solve import _residual
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _need_gpu():
+    if native.device_count() < 1:
+        pytest.fail("no CUDA device visible: the GPU tests need a B200")
+
+
+def _solve(system, eps=1e-12, max_iter=1000, x0=None):
+    import torch
+    ny, nx = system[0].shape
+    bufs = [torch.from_numpy(a.ravel().copy()).cuda() for a in system]
+    x = torch.zeros(nx * ny, dtype=torch.float64, device="cuda") if x0 is None else \
+        torch.from_numpy(x0.ravel().copy()).cuda()
+    torch.cuda.synchronize()
+    its, rel = native.cg_solve_noalloc(nx, ny, *[t.data_ptr() for t in bufs], x.data_ptr(), eps, max_iter,
+                                       x0_from_x=x0 is not None)
+    return x.cpu().numpy().reshape(ny, nx), its, rel
+
+
+def _signed_system(nx, ny):
+    """Couplings of both signs; Ct is 1 plus the sum of their magnitudes."""
+    rng = np.random.default_rng([nx, ny, 1])
+    Gx, Gy = rng.uniform(-1, 1, (ny, nx)), rng.uniform(-1, 1, (ny, nx))
+    Gx[:, -1] = 0
+    Gy[-1] = 0
+    Ct = 1 + np.abs(Gx) + np.abs(Gy)
+    Ct[:, 1:] += np.abs(Gx[:, :-1])
+    Ct[1:] += np.abs(Gy[:-1])
+    return np.where(rng.random((ny, nx)) < 0.1, -Ct, Ct), Gx, Gy, rng.standard_normal((ny, nx))
+
+
+@pytest.mark.parametrize("nx,ny", [(3, 2), (65, 17), (130, 1200), (512, 512), (24, 10922)])
+def test_couplings_of_both_signs(nx, ny):
+    system = _signed_system(nx, ny)
+    x, its, rel = _solve(system)
+    assert 0 < its < 100 and rel < 1e-12
+    assert np.linalg.norm(_residual(*system, x)) <= 1.2e-12 * np.linalg.norm(system[3])
