@@ -42,6 +42,7 @@
 #define FREHD_CG_RES_CUH
 
 #include "cg_common.cuh"
+#include "cg_limit.h"
 #include "cg_res.h"
 
 namespace frehd {
@@ -731,21 +732,6 @@ __device__ __forceinline__ void res_sweep32(const ResCtx &c, ResTile<float, KR> 
       t.x[k][q] = t.x[k][q] + alpha * t.p[k][q];
     }
   }
-}
-
-// The stopping rule (rtc.c:53: ||r|| < eps ||b||, or 1 + ||r|| = 1 for b = 0) as a
-// bound on ||r||^2: the largest double whose root meets it (-1: none does), so that
-// no iteration takes a root and every decision is the rule's own.
-__device__ __forceinline__ double res_limit(double bnorm, double eps) {
-  const double c = eps * bnorm;
-  auto holds = [&](double rr) {
-    const double rn = sqrt(rr);
-    return rn < c || (bnorm == 0.0 && 1.0 + rn == 1.0);
-  };
-  double t = bnorm == 0.0 ? 0x1p-106 : c * c;
-  while (holds(t)) t = __longlong_as_double(__double_as_longlong(t) + 1);
-  while (t > 0.0 && !holds(t)) t = __longlong_as_double(__double_as_longlong(t) - 1);
-  return holds(t) ? t : -1.0;
 }
 
 // The CTA's place in the solve and the first tag; false after an error.  sh and

@@ -49,3 +49,17 @@ def test_couplings_of_both_signs(nx, ny):
     x, its, rel = _solve(system)
     assert 0 < its < 100 and rel < 1e-12
     assert np.linalg.norm(_residual(*system, x)) <= 1.2e-12 * np.linalg.norm(system[3])
+
+
+def test_a_tolerance_no_residual_meets():
+    """eps <= 0 in a domain's configuration: the solve stops at maxIter, a warning."""
+    from frehdc_b200 import deck as D
+    d = D.make_deck(D.DeckSpec(nx=70, ny=40, steps=4, seed=6))
+    for eps in (0.0, -1e-12):
+        cfg = dict(D.config_dict(d), eps=eps, maxIter=5)
+        g = native.Domain(cfg, 0)
+        g.set_fine_bottoms(d.zf, d.r)
+        g.set_tide(D.tide_series(d))
+        g.init(d.bottom, d.bottomXP, d.bottomYP, d.surf0, None, None, d.S0)
+        assert g.step(1) == 5  # FREHD_ERR_CG_NOCONVERGE
+        assert g.stats()["cg_iters"] == 5 and g.stats()["cg_noconverge"] == 1
