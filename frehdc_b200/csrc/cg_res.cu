@@ -81,18 +81,21 @@ template <int KR, bool kMix, class F>
 __device__ __forceinline__ void res_kernel(Scratch *sc, int mixed, double eps_inner, int nb, int csize, F fill) {
   extern __shared__ __align__(16) double res_sm[];
   __shared__ ResSys s;
+  __shared__ int s_run;
   if (csize > 1) {
     // the inbox carries no tag before a neighbour may write to it
     uint4 *in = reinterpret_cast<uint4 *>(res_sm + kResSums * kResThreads + 3 * res_arr(KR));
     for (int e = threadIdx.x; e < res_inbox(KR); e += kResThreads) in[e] = make_uint4(0, 0, 0, 0);
     res_cluster_sync();
   }
-  // (a step that has failed is skipped, but no CTA leaves its cluster early)
-  if ((int)blockIdx.x < nb && *(volatile int *)&sc->status == FREHD_OK) {
-    if (threadIdx.x == 0) fill(&s);
-    __syncthreads();
-    res_solve<KR, kMix, !kMix>(&s, mixed, eps_inner, blockIdx.x, nb, csize);
+  // (a step that has failed is skipped, but no CTA leaves its cluster early; one thread
+  // looks, since another CTA of this solve may set the status meanwhile)
+  if (threadIdx.x == 0) {
+    s_run = (int)blockIdx.x < nb && *(volatile int *)&sc->status == FREHD_OK;
+    if (s_run) fill(&s);
   }
+  __syncthreads();
+  if (s_run) res_solve<KR, kMix, !kMix>(&s, mixed, eps_inner, blockIdx.x, nb, csize);
   // no store into this CTA's shared memory is on its way any more
   if (csize > 1) res_cluster_sync();
 }

@@ -50,6 +50,7 @@ namespace frehd {
 struct ResShared {
   double tot[kResSlot];
   double inv_gamma;  // 1 / (r~, r~) of the last sweep, formed while the sums travel
+  unsigned tag;      // the tag the solve starts from
   int ok;
 };
 
@@ -748,8 +749,12 @@ __device__ __forceinline__ bool res_enter(const ResSys &s, unsigned rank, unsign
   c->slots = s.xbuf;
   c->edges = s.xbuf + 2L * nb * kResSlot + 2L * kResSlot * kResMaxGroups;
   __syncthreads();
-  if (threadIdx.x == 0) sh->ok = 1;
-  c->tag = *(volatile unsigned *)&s.sc->res_tag;
+  if (threadIdx.x == 0) {  // (a CTA that gave up may raise the tag meanwhile)
+    sh->ok = 1;
+    sh->tag = *(volatile unsigned *)&s.sc->res_tag;
+  }
+  __syncthreads();
+  c->tag = sh->tag;
   if (c->tag < 0xC0000000u) return true;
   // the tags near their end: every entry cleared, and the count starts again
   const long all = res_entries(nb, KR);

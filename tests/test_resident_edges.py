@@ -63,3 +63,23 @@ def test_a_tolerance_no_residual_meets():
         g.init(d.bottom, d.bottomXP, d.bottomYP, d.surf0, None, None, d.S0)
         assert g.step(1) == 5  # FREHD_ERR_CG_NOCONVERGE
         assert g.stats()["cg_iters"] == 5 and g.stats()["cg_noconverge"] == 1
+
+
+@pytest.mark.parametrize("nx,ny,skip", [(48, 40, 2), (300, 60, 19), (300, 300, 94)])
+def test_waits_that_run_out_while_other_ctas_start(nx, ny, skip):
+    """The shortest waits, so that CTAs give up and fail the step while others of the
+    same solve still read its status: every such step ends with the timeout's status,
+    and after a new state the domain steps as a fresh one."""
+    from frehdc_b200 import deck as D
+    d = D.make_deck(D.DeckSpec(nx=nx, ny=ny, steps=40, seed=8, dry_frac=0.2))
+    init = (d.bottom, d.bottomXP, d.bottomYP, d.surf0, None, None, d.S0)
+    g, fresh = native.domain_from_deck(d), native.domain_from_deck(d)
+    for _ in range(30):
+        g.set_wait_test(1, skip_barrier_rank=skip)
+        with pytest.raises(native.FrehdError) as e:
+            g.step(1)
+        assert e.value.status == 7  # FREHD_ERR_TIMEOUT
+        g.init(*init)
+    assert g.run(1, 3) == 0 and fresh.run(1, 3) == 0
+    for f in ("surf", "uuXP", "vvYP", "S"):
+        assert np.array_equal(g.download([f])[f], fresh.download([f])[f]), f
