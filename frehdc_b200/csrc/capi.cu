@@ -193,6 +193,10 @@ __global__ void k_set_wait_test(Scratch *sc, unsigned long long limit_ns, int sk
   sc->skip_barrier_rank1 = skip_rank1;
 }
 
+__global__ void k_raise_tag(Scratch *sc, unsigned tag) {
+  if (sc->res_tag < tag) sc->res_tag = tag;
+}
+
 // host copies in the reference layout: index helpers (map.c:45-143)
 struct RefMap {
   int nx, ny;
@@ -256,7 +260,7 @@ long long take_noconv(frehd_domain *d) {
 int launch_cg(frehd_domain *d, const View &w) {
   // a domain whose solver state fits on chip keeps it there
   if (d->cg_schedule == FREHD_CG_SINGLE_SWEEP && d->res_rows)
-    return cgr_launch(w, d->res_rows, d->res_clustered, d->x0_mode, d->eliminate, d->stream);
+    return cgr_launch(w, d->res_rows, d->res_clustered, d->res_plain != 0, d->x0_mode, d->eliminate, d->stream);
   if (d->cg_schedule == FREHD_CG_SINGLE_SWEEP)
     return cg1_launch(w, d->cg1_maps_dev, d->cg1_blocks_n, d->x0_mode, d->eliminate, d->stream);
   View wv = w;
@@ -1033,6 +1037,17 @@ extern "C" int frehd_domain_set_wait_test(frehd_domain *d, long long wait_limit_
   CUDA_TRY(cudaSetDevice(d->device));
   k_set_wait_test<<<1, 1, 0, d->stream>>>(d->sc, (unsigned long long)wait_limit_ns,
                                           skip_barrier_rank + 1);
+  CUDA_TRY(cudaGetLastError());
+  CUDA_TRY(cudaStreamSynchronize(d->stream));
+  return FREHD_OK;
+}
+
+extern "C" int frehd_domain_set_solve_test(frehd_domain *d, int plain_launch, unsigned first_tag) {
+  if (d && d->in_batch) return fail(FREHD_ERR_STATE, "the domain is stepped by a batch (release it first)");
+  if (!d) return fail(FREHD_ERR_INVALID, "bad argument");
+  CUDA_TRY(cudaSetDevice(d->device));
+  d->res_plain = plain_launch;
+  if (first_tag) k_raise_tag<<<1, 1, 0, d->stream>>>(d->sc, first_tag);
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaStreamSynchronize(d->stream));
   return FREHD_OK;

@@ -75,13 +75,26 @@ __device__ __forceinline__ void res_solve(const ResSys *sp, int mixed, double ep
 
 }  // namespace
 
+// Whether this launch stands in clusters of csize, block b being CTA b % csize of its
+// own: as the hardware says, whatever the launch asked for.  (A profiler's replay of a
+// cooperative launch in clusters may come without them, and a store to a CTA that the
+// cluster does not have is a fault.)
+__device__ __forceinline__ bool res_in_clusters(int csize) {
+  unsigned n, rank;
+  asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n));
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  return n == (unsigned)csize && rank == blockIdx.x % csize;
+}
+
 // nb CTAs solve; the grid is a multiple of the cluster size csize, and the CTAs past
-// nb only keep their clusters whole.  fill(&s): the system, by one thread.
+// nb only keep their clusters whole.  Without the clusters all entries go through L2
+// (the same sums).  fill(&s): the system, by one thread.
 template <int KR, bool kMix, class F>
 __device__ __forceinline__ void res_kernel(Scratch *sc, int mixed, double eps_inner, int nb, int csize, F fill) {
   extern __shared__ __align__(16) double res_sm[];
   __shared__ ResSys s;
   __shared__ int s_run;
+  if (csize > 1 && !res_in_clusters(csize)) csize = 1;
   if (csize > 1) {
     // the inbox carries no tag before a neighbour may write to it
     uint4 *in = reinterpret_cast<uint4 *>(res_sm + kResSums * kResThreads + 3 * res_arr(KR));
@@ -247,7 +260,9 @@ namespace {
 
 // Kernel fn on the nb tiles of a solve, cooperatively and, where that fits, in clusters
 // (args: pointers to the kernel's own arguments; nb and the cluster size follow them).
-int launch_solve(void *fn, std::vector<void *> args, int nx, int ny, int rows, int clustered, cudaStream_t stream) {
+// plain: the clusters are announced to the kernel but not asked for.
+int launch_solve(void *fn, std::vector<void *> args, int nx, int ny, int rows, int clustered, bool plain,
+                 cudaStream_t stream) {
   int nb = (int)res_tiles(nx, ny, rows), csize = nb <= kResFlat ? nb : res_group(nb);
   if (nb > clustered) csize = 1;
   args.push_back(&nb);
@@ -264,7 +279,7 @@ int launch_solve(void *fn, std::vector<void *> args, int nx, int ny, int rows, i
   cfg.dynamicSmemBytes = res_smem(rows);
   cfg.stream = stream;
   cfg.attrs = at;
-  cfg.numAttrs = csize > 1 ? 2 : 1;
+  cfg.numAttrs = csize > 1 && !plain ? 2 : 1;
   const cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args.data());
   if (e != cudaSuccess) return fail(FREHD_ERR_CUDA, "resident solve launch: %s", cudaGetErrorString(e));
   return FREHD_OK;
@@ -272,15 +287,16 @@ int launch_solve(void *fn, std::vector<void *> args, int nx, int ny, int rows, i
 
 }  // namespace
 
-int cgr_launch(const View &w, int rows, int clustered, int x0_surface, int eliminate, cudaStream_t stream) {
+int cgr_launch(const View &w, int rows, int clustered, bool plain, int x0_surface, int eliminate,
+               cudaStream_t stream) {
   View wv = w;
   return launch_solve(single_fn(rows, w.p.mixed != 0), {&wv, &x0_surface, &eliminate}, w.gr.nx, w.gr.ny, rows,
-                      clustered, stream);
+                      clustered, plain, stream);
 }
 
 int cgr_launch_sys(const ResSys &s, int rows, int clustered, cudaStream_t stream) {
   ResSys sv = s;
-  return launch_solve(sys_fn(rows), {&sv}, s.nx, s.ny, rows, clustered, stream);
+  return launch_solve(sys_fn(rows), {&sv}, s.nx, s.ny, rows, clustered, false, stream);
 }
 
 int cgr_launch_batch(const View *views2, const int *job_start, const CgJob *jobs, const CgJob *singles,

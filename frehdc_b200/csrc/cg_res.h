@@ -68,8 +68,10 @@ struct ResSys {
 int cgr_capacity(int device, int *ctas, int *clustered);
 // Exchange bytes of a domain's solve with `rows` rows per thread or more.
 long long cgr_exchange_bytes(const Grid &g, int rows);
-// The domain's solve on its own (rows from res_rows of the capacity).
-int cgr_launch(const View &w, int rows, int clustered, int x0_surface, int eliminate, cudaStream_t stream);
+// The domain's solve on its own (rows from res_rows of the capacity).  plain: without the
+// clusters that the kernel expects (frehd_domain_set_solve_test).
+int cgr_launch(const View &w, int rows, int clustered, bool plain, int x0_surface, int eliminate,
+               cudaStream_t stream);
 // The same for a system in any layout, in FP64.  s.xbuf: res_entries of its tiles, no
 // entry of which carries a tag above s.sc->res_tag.
 int cgr_launch_sys(const ResSys &s, int rows, int clustered, cudaStream_t stream);

@@ -63,6 +63,7 @@ struct frehd_domain {
   int res_clustered = 0;         // and how many of them in clusters
   int res_rows = 0;              // its rows per thread (0: the domain does not fit it)
   uint4 *xch = nullptr;          // its exchange entries
+  int res_plain = 0;             // launch it without clusters (frehd_domain_set_solve_test)
   int geom_set = 0, ready = 0;
   frehd_step_stats last{};
   std::vector<void *> allocs;

@@ -183,6 +183,7 @@ def _declare_domain(L: C.CDLL) -> None:
     L.frehd_domain_step.argtypes = [_vp, C.c_int]
     L.frehd_domain_run.argtypes = [_vp, C.c_int, C.c_int]
     L.frehd_domain_set_wait_test.argtypes = [_vp, C.c_longlong, C.c_int]
+    L.frehd_domain_set_solve_test.argtypes = [_vp, C.c_int, C.c_uint]
     L.frehd_domain_phase.argtypes = [_vp, C.c_int, C.c_int, _dp]
     L.frehd_domain_download_system.argtypes = [_vp] + [_dp] * 6
     L.frehd_domain_download_solution.argtypes = [_vp, _dp]
@@ -396,6 +397,12 @@ class Domain:
         barrier so that the others' wait runs out."""
         check(lib().frehd_domain_set_wait_test(self.h, int(wait_limit_ns), int(skip_barrier_rank)),
               "frehd_domain_set_wait_test")
+
+    def set_solve_test(self, plain_launch: bool = False, first_tag: int = 0):
+        """Testing of the on-chip solve (frehd_domain_set_solve_test): a launch without
+        the clusters its kernel is told of, and its exchange counter raised to first_tag."""
+        check(lib().frehd_domain_set_solve_test(self.h, int(plain_launch), int(first_tag)),
+              "frehd_domain_set_solve_test")
 
     def stats(self) -> dict:
         s = StepStats()

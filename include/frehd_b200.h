@@ -258,6 +258,13 @@ int frehd_domain_run(frehd_domain *d, int t0, int nsteps);
  * barrier.  frehd_domain_upload_state / frehd_domain_init clear both settings
  * together with the status. */
 int frehd_domain_set_wait_test(frehd_domain *d, long long wait_limit_ns, int skip_barrier_rank);
+/* Testing of the solve that keeps a small domain on chip (no counterpart in the
+ * reference).  plain_launch != 0: its kernel is told of thread-block clusters but
+ * launched without them, as a profiler's replay may do; it has to notice and
+ * exchange everything through L2, with the same results.  first_tag != 0: its
+ * exchange counter is raised to that value (it only grows; near 2^32 the solve
+ * starts it again), which otherwise takes hours of solving. */
+int frehd_domain_set_solve_test(frehd_domain *d, int plain_launch, unsigned first_tag);
 
 /* Phases of one step, for parity testing against the reference's functions:
  *   FREHD_PHASE_EXPLICIT  solveSourceTerm + matrixCoeffSub/adjust*Boundary (nssolve.c:121-166)

@@ -83,3 +83,21 @@ def test_waits_that_run_out_while_other_ctas_start(nx, ny, skip):
     assert g.run(1, 3) == 0 and fresh.run(1, 3) == 0
     for f in ("surf", "uuXP", "vvYP", "S"):
         assert np.array_equal(g.download([f])[f], fresh.download([f])[f]), f
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("nx,ny", [(48, 40), (130, 500), (520, 500)])
+def test_launched_without_its_clusters(nx, ny, precision):
+    """A launch that does not form the clusters its kernel is told of (one cluster,
+    groups of eight, tall tiles): everything goes through L2, with the same doubles."""
+    from frehdc_b200 import deck as D
+    d = D.make_deck(D.DeckSpec(nx=nx, ny=ny, steps=8, seed=12, dry_frac=0.2))
+    prec = native.PRECISION_MIXED if precision == "mixed" else native.PRECISION_FP64
+    out = []
+    for plain in (False, True):
+        g = native.domain_from_deck(d, precision=prec)
+        g.set_solve_test(plain_launch=plain)
+        assert g.run(1, 4) == 0
+        out.append(g.download(["surf", "uuXP", "vvYP", "S"]))
+    for f in out[0]:
+        assert np.array_equal(out[0][f], out[1][f]), f
