@@ -164,12 +164,25 @@ __device__ __forceinline__ uint4 *res_top(const ResCtx &c, unsigned g, int m) {
   return c.slots + 2L * c.nb * kResSlot + ((c.tag & 1) * kResSlot + m) * kResMaxGroups + g;
 }
 
+// Between what a warp's lanes have read and what any of them passes on.
+__device__ __forceinline__ void res_relay_fence() {
+  __threadfence();
+  __syncwarp();
+  __threadfence();
+}
+
 // The CTAs' sums t of value m, added up: by the whole of one warp, the same total in
 // every CTA.  Up to kResFlat CTAs in one tree over the ranks, else by groups of
 // res_group(nb) and then over the groups.
+// kFence: what the CTAs' threads stored in global memory before the reduction is to be
+// read after it.  The entries themselves order nothing, so the warp that sends them
+// fences after the block barrier in front, the relays between reading and passing on,
+// and every warp after its last read.
+template <bool kFence>
 __device__ __forceinline__ double res_exchange(double t, int m, const ResCtx &c) {
   const unsigned lane = threadIdx.x & 31;
   int *ok = &c.sh->ok;
+  if (kFence) __threadfence();
   if (c.nb <= (unsigned)kResFlat) {
     if (c.csize > 1) {
       if (lane < c.nb) res_sts(res_at(res_in_sum(c, m, c.rank), lane), t, c.tag);
@@ -178,6 +191,7 @@ __device__ __forceinline__ double res_exchange(double t, int m, const ResCtx &c)
       if (lane == 0) res_st(res_slot(c, c.rank, m), t, c.tag);
       t = res_wait(lane < c.nb, [&] { return res_ld(res_slot(c, lane, m)); }, c.tag, c.sc, ok);
     }
+    if (kFence) __threadfence();
     return res_warp_total(t);
   }
   const unsigned group = res_group(c.nb), groups = (c.nb + group - 1) / group;
@@ -185,14 +199,18 @@ __device__ __forceinline__ double res_exchange(double t, int m, const ResCtx &c)
     const unsigned mine = c.rank % group, g = c.rank / group, members = min(group, c.nb - g * group);
     if (mine) {  // to the group's first CTA, and the total back
       if (lane == 0) res_sts(res_at(res_in_sum(c, m, mine), 0), t, c.tag);
-      return res_wait(true, [&] { return res_lds(res_in_total(c, m)); }, c.tag, c.sc, ok);
+      t = res_wait(true, [&] { return res_lds(res_in_total(c, m)); }, c.tag, c.sc, ok);
+      if (kFence) __threadfence();
+      return t;
     }
     const double own = t;
     t = res_wait(lane > 0 && lane < members, [&] { return res_lds(res_in_sum(c, m, lane)); }, c.tag, c.sc, ok);
     t = res_warp_total(lane == 0 ? own : t);
+    if (kFence) res_relay_fence();
     if (lane == 0) res_st(res_top(c, g, m), t, c.tag);
     t = res_wait(lane < groups, [&] { return res_ld(res_top(c, lane, m)); }, c.tag, c.sc, ok);
     t = res_warp_total(t);
+    if (kFence) res_relay_fence();
     if (lane > 0 && lane < members) res_sts(res_at(res_in_total(c, m), lane), t, c.tag);
     return t;
   }
@@ -223,6 +241,7 @@ __device__ __forceinline__ double res_exchange(double t, int m, const ResCtx &c)
     const double x = __shfl_sync(0xffffffffu, v, (lane % per) * group);
     if (lane / per == r0 / 32) t = x;
   }
+  if (kFence) __threadfence();
   return res_warp_total(!grouped || lane < groups ? t : 0.0);
 }
 
@@ -230,7 +249,7 @@ __device__ __forceinline__ double res_exchange(double t, int m, const ResCtx &c)
 // thread), and a barrier among them for the entries stored before it under this tag
 // (the caller has advanced it).  Warp m sums value m, in the CTA and over the CTAs;
 // `meanwhile` runs in the others.  False after a wait that gave up.
-template <int NV, class M>
+template <int NV, bool kFence = false, class M>
 __device__ __forceinline__ bool res_allreduce(double (&v)[kResSums], const ResCtx &c, M meanwhile) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   ResShared *sh = c.sh;
@@ -250,7 +269,7 @@ __device__ __forceinline__ bool res_allreduce(double (&v)[kResSums], const ResCt
 #pragma unroll
       for (int q = 0; q < n; ++q) part[q] += part[q + n];
     double t = res_warp_total(part[0]);
-    if (c.nb > 1) t = res_exchange(t, wid, c);
+    if (c.nb > 1) t = res_exchange<kFence>(t, wid, c);
     if (lane == 0) sh->tot[wid] = t;
   } else {
     meanwhile(); }
@@ -1080,13 +1099,12 @@ __device__ __forceinline__ int res_mixed(const ResSys &s, double eps_inner, unsi
           s.x[kk] = xd[k][q];
         }
       }
-    __threadfence();
+    // (x by this CTA's threads, before the block barrier; the neighbours' after it)
     ++c.tag;
-    if (!res_allreduce<1>(red, c, [] {})) {
+    if (!res_allreduce<1, true>(red, c, [] {})) {
       ret = 0;
       break;
     }
-    __threadfence();
   }
   if (ret == 1) {
     if (it_all == 0) {  // converged at the start: x was never stored

@@ -101,3 +101,22 @@ def test_launched_without_its_clusters(nx, ny, precision):
         out.append(g.download(["surf", "uuXP", "vvYP", "S"]))
     for f in out[0]:
         assert np.array_equal(out[0][f], out[1][f]), f
+
+
+@pytest.mark.parametrize("nx,ny", [(64, 250), (130, 900), (500, 540)])
+def test_refinements_read_their_neighbours_new_x(nx, ny):
+    """A tight tolerance, so that x passes between the tiles several times: the same
+    doubles in every run, and the FP64 solution within the refinement's own bound."""
+    from frehdc_b200 import deck as D
+    d = D.make_deck(D.DeckSpec(nx=nx, ny=ny, steps=4, seed=33, dry_frac=0.2, eps=1e-13))
+
+    def solution(precision, eps_inner):
+        g = native.domain_from_deck(d, precision=precision, eps_inner=eps_inner)
+        g.phase(native.PHASE_EXPLICIT, 1)
+        g.phase(native.PHASE_SOLVE, 1)
+        return g.solution()
+    want = solution(native.PRECISION_FP64, 1e-5)
+    first = solution(native.PRECISION_MIXED, 1e-3)
+    assert np.max(np.abs(first - want)) <= 1e-10 * np.max(np.abs(want))  # the solve tests' bound
+    for _ in range(10):
+        assert np.array_equal(solution(native.PRECISION_MIXED, 1e-3), first)
