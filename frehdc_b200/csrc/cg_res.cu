@@ -33,7 +33,7 @@ __device__ __forceinline__ void sys_of(const View &w, int x0_surface, int elimin
 // other tile heights they must not share a register allocation (the inlined FP32
 // sweeps of 64 x 64 tiles spilled 2.6 KB).
 template <int KR>
-__device__ __noinline__ int res_job_mixed(const ResSys *sp, double eps_inner, unsigned rank, unsigned nb,
+__device__ __noinline__ ResEnd res_job_mixed(const ResSys *sp, double eps_inner, unsigned rank, unsigned nb,
                                           unsigned csize) {
   extern __shared__ __align__(16) double res_sm[];
   __shared__ ResShared sh;
@@ -41,11 +41,12 @@ __device__ __noinline__ int res_job_mixed(const ResSys *sp, double eps_inner, un
   return res_mixed<KR>(s, eps_inner, rank, nb, csize, res_sm, &sh);
 }
 template <int KR>
-__device__ __noinline__ bool res_job_fp64(const ResSys *sp, unsigned rank, unsigned nb, unsigned csize) {
+__device__ __noinline__ bool res_job_fp64(const ResSys *sp, unsigned rank, unsigned nb, unsigned csize,
+                                          unsigned from) {
   extern __shared__ __align__(16) double res_sm[];
   __shared__ ResShared sh;
   const ResSys s = *sp;
-  return res_fp64<KR>(s, rank, nb, csize, res_sm, &sh);
+  return res_fp64<KR>(s, rank, nb, csize, from, res_sm, &sh);
 }
 
 // The domain's solve in its configured precision by nb CTAs (in clusters of csize); sp
@@ -59,17 +60,18 @@ __device__ __forceinline__ void res_solve(const ResSys *sp, int mixed, double ep
     return;
   }
   if (kMix && mixed) {
-    if (res_job_mixed<KR>(sp, eps_inner, rank, nb, csize) != 2) return;
-    if (res_job_fp64<KR>(sp, rank, nb, csize) && rank == 0 && threadIdx.x == 0) sp->sc->cg_fallback = 2;
+    const ResEnd end = res_job_mixed<KR>(sp, eps_inner, rank, nb, csize);
+    if (end.code != 2) return;
+    if (res_job_fp64<KR>(sp, rank, nb, csize, end.tag) && rank == 0 && threadIdx.x == 0) sp->sc->cg_fallback = 2;
     return;
   }
   if (kAlone) {
     extern __shared__ __align__(16) double res_sm[];
     __shared__ ResShared sh;
     const ResSys s = *sp;
-    res_fp64<KR>(s, rank, nb, csize, res_sm, &sh);
+    res_fp64<KR>(s, rank, nb, csize, 0, res_sm, &sh);
   } else {
-    res_job_fp64<KR>(sp, rank, nb, csize);
+    res_job_fp64<KR>(sp, rank, nb, csize, 0);
   }
 }
 

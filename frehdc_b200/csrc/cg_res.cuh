@@ -69,6 +69,10 @@ struct ResCtx {
 
 namespace {
 
+// From this tag on a solve first clears its entries and starts again at 0: a quarter of
+// the numbers are left for the reductions of that solve's launch.
+constexpr unsigned kResTagEnd = 0xC0000000u;
+
 __device__ __forceinline__ uint4 res_ld(const uint4 *a) {
   uint4 v;
   asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
@@ -754,10 +758,19 @@ __device__ __forceinline__ void res_sweep32(const ResCtx &c, ResTile<float, KR> 
   }
 }
 
-// The CTA's place in the solve and the first tag; false after an error.  sh and
-// the dynamic shared memory belong to the caller's CTA.
+// What a mixed solve leaves: 0 after an error, 1 when done, 2 when the FP64 solve must
+// take over, from the tag it ended with.
+struct ResEnd {
+  int code;
+  unsigned tag;
+};
+
+// The CTA's place in the solve and the first tag: the domain's, or `from` if a solve of
+// the same launch goes on from there (its other CTAs may not have read the domain's yet
+// when this one leaves, so the two solves enter and leave once).  False after an error.
+// sh and the dynamic shared memory belong to the caller's CTA.
 __device__ __forceinline__ bool res_enter(const ResSys &s, unsigned rank, unsigned nb, unsigned csize, int KR,
-                                          double *sm, ResShared *sh, ResCtx *c) {
+                                          unsigned from, double *sm, ResShared *sh, ResCtx *c) {
   c->rank = rank;
   c->nb = nb;
   c->csize = csize;
@@ -770,24 +783,25 @@ __device__ __forceinline__ bool res_enter(const ResSys &s, unsigned rank, unsign
   __syncthreads();
   if (threadIdx.x == 0) {  // (a CTA that gave up may raise the tag meanwhile)
     sh->ok = 1;
-    sh->tag = *(volatile unsigned *)&s.sc->res_tag;
+    sh->tag = from ? from : *(volatile unsigned *)&s.sc->res_tag;
   }
   __syncthreads();
   c->tag = sh->tag;
-  if (c->tag < 0xC0000000u) return true;
+  if (from || c->tag < kResTagEnd) return true;
   // the tags near their end: every entry cleared, and the count starts again
   const long all = res_entries(nb, KR);
   for (long e = (long)rank * kResThreads + threadIdx.x; e < all; e += (long)nb * kResThreads)
     s.xbuf[e] = make_uint4(0, 0, 0, 0);
-  __threadfence();
   __syncthreads();
   if (nb > 1) {
     // a plain arrival count (all CTAs are co-resident), bounded like every wait
     if (threadIdx.x == 0) {
+      const unsigned long long lim = s.sc->wait_limit_ns ? s.sc->wait_limit_ns : kBarrierTimeoutNs;
       const unsigned long long t0 = gtimer_ns();
+      __threadfence();
       atomicAdd(&s.sc->bar_count, 1u);
       while (*(volatile unsigned *)&s.sc->bar_count < nb)
-        if (gtimer_ns() - t0 > kBarrierTimeoutNs) {
+        if (gtimer_ns() - t0 > lim) {
           set_status(s.sc, FREHD_ERR_TIMEOUT);
           sh->ok = 0;
           break;
@@ -804,7 +818,7 @@ __device__ __forceinline__ bool res_enter(const ResSys &s, unsigned rank, unsign
 // The solve's last act in each CTA.
 __device__ __forceinline__ void res_leave(const ResSys &s, const ResCtx &c) {
   if (threadIdx.x != 0) return;
-  if (*(volatile unsigned *)&s.sc->res_tag >= 0xC0000000u && c.tag < 0x40000000u) {
+  if (*(volatile unsigned *)&s.sc->res_tag >= kResTagEnd && c.tag < kResTagEnd) {
     // after a restart of the tags (res_enter): every CTA has read the old one by now
     if (c.rank == 0) {
       s.sc->bar_count = 0;
@@ -816,16 +830,17 @@ __device__ __forceinline__ void res_leave(const ResSys &s, const ResCtx &c) {
 }
 
 // FP64 solve by nb CTAs, of which this one is number `rank` = its tile number.
-// sm: res_smem(KR) bytes of shared memory.  False after an error (status set).
+// sm: res_smem(KR) bytes of shared memory.  from: see res_enter.  False after an error
+// (status set).
 template <int KR>
-__device__ __forceinline__ bool res_fp64(const ResSys &s, unsigned rank, unsigned nb, unsigned csize, double *sm,
-                                         ResShared *sh) {
+__device__ __forceinline__ bool res_fp64(const ResSys &s, unsigned rank, unsigned nb, unsigned csize, unsigned from,
+                                         double *sm, ResShared *sh) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int ntx = res_ntx(s.nx);
   const int i0 = (int)(rank % ntx) * kResTW, j0 = (int)(rank / ntx) * res_th(KR);
   double *R = sm + kResSums * kResThreads;
   ResCtx c;
-  if (!res_enter(s, rank, nb, csize, KR, sm, sh, &c)) return false;
+  if (!res_enter(s, rank, nb, csize, KR, from, sm, sh, &c)) return false;
   ResTile<double, KR> t;
   double w[KR][2], as[KR][2];  // A~ r~, A~ p
   // x~ and |Ct| of the tallest tile's cells lie in shared memory (its registers would
@@ -989,10 +1004,9 @@ __device__ __forceinline__ bool res_fp64(const ResSys &s, unsigned rank, unsigne
 // Mixed-precision solve: FP32 inner solves on the resident tile inside FP64
 // refinement (cg1_mixed in cg1.cu, same steps, same stopping rules).  x lives in
 // registers; between two inner solves it goes through global memory, where the
-// next residual reads its neighbours.  0 after an error, 1 when done, 2 when the
-// refinement stalled and the FP64 solve must take over.
+// next residual reads its neighbours.
 template <int KR>
-__device__ __forceinline__ int res_mixed(const ResSys &s, double eps_inner, unsigned rank, unsigned nb, unsigned csize,
+__device__ __forceinline__ ResEnd res_mixed(const ResSys &s, double eps_inner, unsigned rank, unsigned nb, unsigned csize,
                                          double *sm, ResShared *sh) {
   constexpr int kArr = res_arr(KR);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1001,7 +1015,7 @@ __device__ __forceinline__ int res_mixed(const ResSys &s, double eps_inner, unsi
   double *ds = sm + kResSums * kResThreads;
   float *P = reinterpret_cast<float *>(ds), *R = P + kArr;  // the other copies lie 2 kArr further
   ResCtx c;
-  if (!res_enter(s, rank, nb, csize, KR, sm, sh, &c)) return 0;
+  if (!res_enter(s, rank, nb, csize, KR, 0, sm, sh, &c)) return ResEnd{0, 0};
   ResTile<float, KR> t;
   double xd[KR][2];
 #pragma unroll
@@ -1124,8 +1138,8 @@ __device__ __forceinline__ int res_mixed(const ResSys &s, double eps_inner, unsi
       s.sc->cg_bb = bnorm * bnorm;
     }
   }
-  res_leave(s, c);
-  return ret;
+  if (ret != 2) res_leave(s, c);
+  return ResEnd{ret, c.tag};
 }
 
 }  // namespace

@@ -120,3 +120,23 @@ def test_refinements_read_their_neighbours_new_x(nx, ny):
     assert np.max(np.abs(first - want)) <= 1e-10 * np.max(np.abs(want))  # the solve tests' bound
     for _ in range(10):
         assert np.array_equal(solution(native.PRECISION_MIXED, 1e-3), first)
+
+
+@pytest.mark.parametrize("precision,eps", [("fp64", 1e-12), ("mixed", 1e-12), ("mixed", 1e-17)])
+@pytest.mark.parametrize("nx,ny", [(40, 12), (300, 60), (64, 2100)])
+def test_exchange_counter_starts_again(nx, ny, precision, eps):
+    """The exchange counter passes the value from which a solve restarts it, in every
+    step anew: one tile, clusters, and no clusters; with eps = 1e-17 the mixed solve's
+    refinement stalls and its FP64 solve takes over in the same launch."""
+    from frehdc_b200 import deck as D
+    d = D.make_deck(D.DeckSpec(nx=nx, ny=ny, steps=16, seed=14, dry_frac=0.2, eps=eps))
+    prec = native.PRECISION_MIXED if precision == "mixed" else native.PRECISION_FP64
+    g, want = (native.domain_from_deck(d, precision=prec) for _ in range(2))
+    for tt in range(1, 13):
+        g.set_solve_test(first_tag=0xC0000000 - 5 * tt)
+        assert g.step(tt) == want.step(tt) == 0
+        assert g.step(tt + 12) == want.step(tt + 12) == 0  # from beyond the bound
+        if eps < 1e-16:
+            assert g.stats()["cg_fallback"] == 2
+    for f in ("surf", "uuXP", "vvYP", "S"):
+        assert np.array_equal(g.download([f])[f], want.download([f])[f]), f
