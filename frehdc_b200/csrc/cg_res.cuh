@@ -49,7 +49,6 @@ namespace frehd {
 
 struct ResShared {
   double tot[kResSlot];
-  double inv_gamma;  // 1 / (r~, r~) of the last sweep, formed while the sums travel
   unsigned tag;      // the tag the solve starts from
   int ok;
 };
@@ -904,7 +903,7 @@ __device__ __forceinline__ bool res_fp64(const ResSys &s, unsigned rank, unsigne
     red[3] = first[1];
     ++c.tag;
     if (!(ok = res_allreduce<4>(red, c, [] {}))) break;
-    double gamma = red[0], delta = red[3], e1 = 0.0, e2 = 0.0, e3 = 0.0;
+    double gamma = red[0], gamma_old = 1.0, delta = red[3], e1 = 0.0, e2 = 0.0, e3 = 0.0;
     rr = red[1];
     bnorm = sqrt(red[2]);
     limit = res_limit(bnorm, s.eps);
@@ -913,7 +912,7 @@ __device__ __forceinline__ bool res_fp64(const ResSys &s, unsigned rank, unsigne
     bool stalled = false;
     it = 0;
     while (!(rr <= limit) && it < s.max_iter) {
-      const double beta = it == 0 ? 0.0 : gamma * sh->inv_gamma;
+      const double beta = it == 0 ? 0.0 : gamma / gamma_old;
       const double alpha = gamma / (delta + beta * (e1 + e2) + beta * beta * e3);
       ++it;
       ++c.tag;
@@ -950,11 +949,11 @@ __device__ __forceinline__ bool res_fp64(const ResSys &s, unsigned rank, unsigne
         }
       }
       ok = res_allreduce<6>(red, c, [&] {
-        if (wid == kResSums) sh->inv_gamma = 1.0 / gamma;
         res_ring_take<double, KR>(c, t);
         ring_stencil();
       });
       if (!ok) break;
+      gamma_old = gamma;
       gamma = red[0];
       delta = red[1];
       e1 = red[2];
@@ -1069,25 +1068,23 @@ __device__ __forceinline__ ResEnd res_mixed(const ResSys &s, double eps_inner, u
     if (outer > 0 && rr > 1e-2 * rr_prev) break;  // no tenfold gain: FP64 takes over
     rr_prev = rr;
     // A~ d~ = r~ until (r~, r~) fell by eps_inner^2
-    double gamma = red[0], delta = red[3], e1 = 0.0, e2 = 0.0, e3 = 0.0;
+    double gamma = red[0], gamma_old = 1.0, delta = red[3], e1 = 0.0, e2 = 0.0, e3 = 0.0;
     const double stop = eps_inner * eps_inner * gamma;
 #pragma unroll
     for (int k = 0; k < KR; ++k) t.x[k][0] = t.x[k][1] = 0.0f;
     int it = 0;
     bool ok = true;
     while (gamma > stop && it < s.max_iter) {
-      const double beta = it == 0 ? 0.0 : gamma * sh->inv_gamma;
+      const double beta = it == 0 ? 0.0 : gamma / gamma_old;
       const double alpha = gamma / (delta + beta * (e1 + e2) + beta * beta * e3);
       const int cur = it & 1;
       ++it;
       ++c.tag;
       res_sweep32<KR>(c, t, P + 2 * cur * kArr, R + 2 * cur * kArr, P + 2 * (cur ^ 1) * kArr,
                       R + 2 * (cur ^ 1) * kArr, (float)alpha, (float)beta, p2, red);
-      ok = res_allreduce<5>(red, c, [&] {
-        if (wid == kResSums) sh->inv_gamma = 1.0 / gamma;
-        res_ring_take<float, KR>(c, t);
-      });
+      ok = res_allreduce<5>(red, c, [&] { res_ring_take<float, KR>(c, t); });
       if (!ok) break;
+      gamma_old = gamma;
       gamma = red[0];
       delta = red[1];
       e1 = red[2];

@@ -140,3 +140,24 @@ def test_exchange_counter_starts_again(nx, ny, precision, eps):
             assert g.stats()["cg_fallback"] == 2
     for f in ("surf", "uuXP", "vvYP", "S"):
         assert np.array_equal(g.download([f])[f], want.download([f])[f]), f
+
+
+@pytest.mark.parametrize("scale", [1e-158, 1e-150, 1.0, 1e140])
+def test_right_hand_sides_of_any_size(scale):
+    """beta = gamma / gamma_old, a quotient of two sums: with b of this size the sums
+    leave the range in which 1 / gamma_old exists.  Scaling b by a power of two scales
+    every number of the solve, so x scales to the last bit where the squares keep all
+    theirs: the last ones are (1e-12)^2 of the first (b above 1e-130)."""
+    rng = np.random.default_rng(21)
+    nx, ny = 130, 70
+    system = list(_signed_system(nx, ny))
+    system[0] = np.abs(system[0])
+    system[3] = rng.standard_normal((ny, nx))
+    ref, its_ref, _ = _solve(system)
+    p2 = 2.0 ** np.round(np.log2(scale))
+    x, its, _ = _solve([*system[:3], system[3] * p2])
+    assert np.all(np.isfinite(x)) and 0 < its
+    if scale > 1e-130:
+        assert its == its_ref and np.array_equal(x, ref * p2)
+    else:  # the sums lose their bits on the way: a solution of a coarser solve
+        assert np.linalg.norm(_residual(*system[:3], system[3] * p2, x) / p2) <= 1e-4 * np.linalg.norm(system[3])
