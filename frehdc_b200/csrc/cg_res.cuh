@@ -985,7 +985,8 @@ __device__ __forceinline__ bool res_fp64(const ResSys &s, unsigned rank, unsigne
       const int lx = e % kResTW, ly = e / kResTW, i = i0 + lx, j = j0 + ly;
       if (res_in(s, i, j)) {
         const long k = s.off + (long)j * s.pitch + i;
-        s.x[k] = R[res_q(lx, ly)] / sqrt(fabs(s.Ct[k]));
+        // (a start that meets the tolerance is the solution, to the last bit)
+        s.x[k] = it_all > 0 ? R[res_q(lx, ly)] / sqrt(fabs(s.Ct[k])) : s.x0 ? s.x0[k] : 0.0;
       }
     }
     if (rank == 0 && threadIdx.x == 0) {

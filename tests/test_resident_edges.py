@@ -161,3 +161,13 @@ def test_right_hand_sides_of_any_size(scale):
         assert its == its_ref and np.array_equal(x, ref * p2)
     else:  # the sums lose their bits on the way: a solution of a coarser solve
         assert np.linalg.norm(_residual(*system[:3], system[3] * p2, x) / p2) <= 1e-4 * np.linalg.norm(system[3])
+
+
+@pytest.mark.parametrize("nx,ny", [(3, 2), (130, 70), (512, 512)])
+def test_a_start_that_meets_the_tolerance_is_returned(nx, ny):
+    """No iteration, no rounding: the caller's x comes back as it was."""
+    system = _signed_system(nx, ny)
+    x, _, _ = _solve(system)
+    again, its, rel = _solve(system, eps=1e-6, x0=x)
+    assert its == 0 and rel < 1e-6
+    assert np.array_equal(again, x)
