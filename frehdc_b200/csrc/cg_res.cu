@@ -1,9 +1,7 @@
 // Kernels of the resident solve (cg_res.cuh): one domain, or many in a batch.
 #include "cg_res.cuh"
 
-#include <map>
 #include <mutex>
-#include <vector>
 
 #include "frehd_internal.h"
 
@@ -213,12 +211,15 @@ int max_clusters(void *fn, unsigned smem, int size) {
 
 int cgr_capacity(int device, int *ctas, int *clustered) {
   // found once per device; domains may be created on several host threads
+  constexpr int kMaxDevices = 64;
   static std::mutex mu;
-  static std::map<int, std::pair<int, int>> known;
+  static struct {
+    int ctas, clustered;
+  } known[kMaxDevices];
   std::lock_guard<std::mutex> lk(mu);
-  if (const auto it = known.find(device); it != known.end()) {
-    *ctas = it->second.first;
-    *clustered = it->second.second;
+  if (device >= 0 && device < kMaxDevices && known[device].ctas) {
+    *ctas = known[device].ctas;
+    *clustered = known[device].clustered;
     return FREHD_OK;
   }
   int nsm = 0, least = 1 << 30, clustered_n = kResClustered;
@@ -245,7 +246,7 @@ int cgr_capacity(int device, int *ctas, int *clustered) {
   if (least < 1) return fail(FREHD_ERR_CUDA, "the resident solve does not fit on an SM");
   *ctas = nsm;  // one CTA per SM: more would share the SM's latency, not hide it
   *clustered = clustered_n;
-  known[device] = {*ctas, *clustered};
+  if (device >= 0 && device < kMaxDevices) known[device] = {*ctas, *clustered};
   return FREHD_OK;
 }
 
@@ -261,14 +262,17 @@ long long cgr_exchange_bytes(const Grid &g, int rows) {
 namespace {
 
 // Kernel fn on the nb tiles of a solve, cooperatively and, where that fits, in clusters
-// (args: pointers to the kernel's own arguments; nb and the cluster size follow them).
+// (own: pointers to the kernel's own arguments; nb and the cluster size follow them).
 // plain: the clusters are announced to the kernel but not asked for.
-int launch_solve(void *fn, std::vector<void *> args, int nx, int ny, int rows, int clustered, bool plain,
+template <int N>
+int launch_solve(void *fn, void *const (&own)[N], int nx, int ny, int rows, int clustered, bool plain,
                  cudaStream_t stream) {
   int nb = (int)res_tiles(nx, ny, rows), csize = nb <= kResFlat ? nb : res_group(nb);
   if (nb > clustered) csize = 1;
-  args.push_back(&nb);
-  args.push_back(&csize);
+  void *args[N + 2];
+  for (int n = 0; n < N; ++n) args[n] = own[n];
+  args[N] = &nb;
+  args[N + 1] = &csize;
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeCooperative;
@@ -282,7 +286,7 @@ int launch_solve(void *fn, std::vector<void *> args, int nx, int ny, int rows, i
   cfg.stream = stream;
   cfg.attrs = at;
   cfg.numAttrs = csize > 1 && !plain ? 2 : 1;
-  const cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args.data());
+  const cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
   if (e != cudaSuccess) return fail(FREHD_ERR_CUDA, "resident solve launch: %s", cudaGetErrorString(e));
   return FREHD_OK;
 }
@@ -292,13 +296,15 @@ int launch_solve(void *fn, std::vector<void *> args, int nx, int ny, int rows, i
 int cgr_launch(const View &w, int rows, int clustered, bool plain, int x0_surface, int eliminate,
                cudaStream_t stream) {
   View wv = w;
-  return launch_solve(single_fn(rows, w.p.mixed != 0), {&wv, &x0_surface, &eliminate}, w.gr.nx, w.gr.ny, rows,
-                      clustered, plain, stream);
+  void *const own[] = {&wv, &x0_surface, &eliminate};
+  return launch_solve(single_fn(rows, w.p.mixed != 0), own, w.gr.nx, w.gr.ny, rows, clustered, plain,
+                      stream);
 }
 
 int cgr_launch_sys(const ResSys &s, int rows, int clustered, cudaStream_t stream) {
   ResSys sv = s;
-  return launch_solve(sys_fn(rows), {&sv}, s.nx, s.ny, rows, clustered, false, stream);
+  void *const own[] = {&sv};
+  return launch_solve(sys_fn(rows), own, s.nx, s.ny, rows, clustered, false, stream);
 }
 
 int cgr_launch_batch(const View *views2, const int *job_start, const CgJob *jobs, const CgJob *singles,
