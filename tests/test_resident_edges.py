@@ -165,9 +165,11 @@ def test_right_hand_sides_of_any_size(scale):
 
 @pytest.mark.parametrize("nx,ny", [(3, 2), (130, 70), (512, 512)])
 def test_a_start_that_meets_the_tolerance_is_returned(nx, ny):
-    """No iteration, no rounding: the caller's x comes back as it was."""
+    """No iteration, no rounding: the caller's x comes back as it was.  (Not the solve's
+    own x: that one is already a quotient by sqrt|Ct|, and the scaling back exact.)"""
     system = _signed_system(nx, ny)
     x, _, _ = _solve(system)
+    x *= 1 + 1e-9 * np.random.default_rng(2).uniform(0.5, 1, x.shape)
     again, its, rel = _solve(system, eps=1e-6, x0=x)
     assert its == 0 and rel < 1e-6
     assert np.array_equal(again, x)
