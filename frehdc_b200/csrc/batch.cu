@@ -208,7 +208,7 @@ int launch_step(frehd_batch *b) {
   int rc = FREHD_OK;
   if (!tl && b->nrctas > 0)
     rc = cgr_launch_batch(b->views2.p, b->rstart.p, b->rjobs.p, b->rsingles.p, b->nrsingles,
-                          &b->bsync.p->taken, b->nrctas, b->any_rmixed, b->stream);
+                          b->bsync.p, b->nrctas, b->any_rmixed, b->stream);
   if (rc) return rc;
   if (b->nctas > 0)
     rc = tl ? cg1_launch_tiles(b->views2.p, b->maps.p, b->bdoms.p, b->bstates.p, b->btiles.p,

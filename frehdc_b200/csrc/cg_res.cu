@@ -25,6 +25,33 @@ __device__ __forceinline__ void sys_of(const View &w, int x0_surface, int elimin
   s->eliminate = eliminate;
   s->sc = w.sc;
   s->xbuf = w.xch;
+  s->beat = nullptr;
+}
+
+// A batched solve's CTAs come to it one by one, each from solves of its own, and a
+// partner may be held up for as long as those take: hundreds of thousands of iterations,
+// or the whole wait of one that gives up.  None of that is this domain's time-out, so
+// its solve starts, and its waits count, once all nb CTAs are there.  That wait ends too:
+// it gives up when no solve of the launch has shown a sign of life (a solve that ends,
+// or kResBeat reductions) for several times the longest that a solve waits in vain.
+__device__ __forceinline__ bool res_arrive(Scratch *sc, unsigned nb, unsigned *beat) {
+  atomicAdd(&sc->res_arrived, 1u);
+  const unsigned long long own = sc->wait_limit_ns;
+  const unsigned long long lim = 5 * (own > kBarrierTimeoutNs ? own : kBarrierTimeoutNs);
+  unsigned seen = *(volatile unsigned *)beat;
+  unsigned long long t0 = gtimer_ns();
+  while (*(volatile unsigned *)&sc->res_arrived < nb) {
+    if (*(volatile int *)&sc->status != FREHD_OK) return false;
+    const unsigned now = *(volatile unsigned *)beat;
+    if (now != seen) {
+      seen = now;
+      t0 = gtimer_ns();
+    } else if (gtimer_ns() - t0 > lim) {
+      set_status(sc, FREHD_ERR_TIMEOUT);
+      return false;
+    }
+  }
+  return *(volatile int *)&sc->status == FREHD_OK;
 }
 
 // The two solves as functions of their own: in one kernel with each other or with
@@ -127,7 +154,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cgr_sys(ResSys sys, int nb, 
 template <bool kMix>
 __global__ void __launch_bounds__(kResThreads, 1)
     k_cgr_batch(const View *__restrict__ views2, const int *__restrict__ job_start,
-                const CgJob *__restrict__ jobs, const CgJob *__restrict__ singles, int nsingles, int *taken) {
+                const CgJob *__restrict__ jobs, const CgJob *__restrict__ singles, int nsingles, Scratch *bsync) {
   __shared__ ResSys s_sys;
   __shared__ double s_eps;
   __shared__ int s_mixed, s_next, s_run;
@@ -138,7 +165,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
       jb = jobs[q0 + n];
     } else {
       __syncthreads();  // every thread read the previous s_next
-      if (threadIdx.x == 0) s_next = atomicAdd(taken, 1);
+      if (threadIdx.x == 0) s_next = atomicAdd(&bsync->taken, 1);
       __syncthreads();
       if (s_next >= nsingles) break;
       jb = singles[s_next];
@@ -148,9 +175,10 @@ __global__ void __launch_bounds__(kResThreads, 1)
       const View *v = views2 + 2 * jb.d;
       v += *(volatile int *)&v->sc->cur;
       sys_of(*v, jb.flags & 1, (jb.flags >> 1) & 1, &s_sys);
+      s_sys.beat = &bsync->beat;
       s_mixed = v->p.mixed;
       s_eps = v->p.eps_inner;
-      s_run = *(volatile int *)&v->sc->status == FREHD_OK;
+      s_run = res_arrive(v->sc, jb.nb, &bsync->beat);
     }
     __syncthreads();
     if (!s_run) continue;
@@ -160,6 +188,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
       case 2: res_solve<2, kMix>(&s_sys, s_mixed, s_eps, jb.rank, jb.nb, 1); break;
       default: res_solve<4, kMix>(&s_sys, s_mixed, s_eps, jb.rank, jb.nb, 1); break;
     }
+    if (threadIdx.x == 0) atomicAdd(&bsync->beat, 1u);
   }
 }
 
@@ -308,8 +337,8 @@ int cgr_launch_sys(const ResSys &s, int rows, int clustered, cudaStream_t stream
 }
 
 int cgr_launch_batch(const View *views2, const int *job_start, const CgJob *jobs, const CgJob *singles,
-                     int nsingles, int *taken, int nctas, int any_mixed, cudaStream_t stream) {
-  void *args[] = {&views2, &job_start, &jobs, &singles, &nsingles, &taken};
+                     int nsingles, Scratch *bsync, int nctas, int any_mixed, cudaStream_t stream) {
+  void *args[] = {&views2, &job_start, &jobs, &singles, &nsingles, &bsync};
   cudaError_t e = cudaLaunchCooperativeKernel(batch_fn(any_mixed != 0), dim3(nctas), dim3(kResThreads), args,
                                               res_smem(kResMaxKR), stream);
   if (e != cudaSuccess) return fail(FREHD_ERR_CUDA, "k_cgr_batch launch: %s", cudaGetErrorString(e));

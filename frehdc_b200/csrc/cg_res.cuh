@@ -49,7 +49,8 @@ namespace frehd {
 
 struct ResShared {
   double tot[kResSlot];
-  unsigned tag;      // the tag the solve starts from
+  unsigned tag;    // the tag the solve starts from
+  unsigned *beat;  // ResSys::beat
   int ok;
 };
 
@@ -71,6 +72,8 @@ namespace {
 // From this tag on a solve first clears its entries and starts again at 0: a quarter of
 // the numbers are left for the reductions of that solve's launch.
 constexpr unsigned kResTagEnd = 0xC0000000u;
+// Reductions between two signs of life of a solve (a few milliseconds).
+constexpr unsigned kResBeat = 1024;
 
 __device__ __forceinline__ uint4 res_ld(const uint4 *a) {
   uint4 v;
@@ -275,7 +278,9 @@ __device__ __forceinline__ bool res_allreduce(double (&v)[kResSums], const ResCt
     if (c.nb > 1) t = res_exchange<kFence>(t, wid, c);
     if (lane == 0) sh->tot[wid] = t;
   } else {
-    meanwhile(); }
+    meanwhile();
+    if (threadIdx.x == kResThreads - 1 && (c.tag & (kResBeat - 1)) == 0 && sh->beat) atomicAdd(sh->beat, 1u);
+  }
   __syncthreads();
 #pragma unroll
   for (int m = 0; m < NV; ++m) v[m] = sh->tot[m];
@@ -782,6 +787,7 @@ __device__ __forceinline__ bool res_enter(const ResSys &s, unsigned rank, unsign
   __syncthreads();
   if (threadIdx.x == 0) {  // (a CTA that gave up may raise the tag meanwhile)
     sh->ok = 1;
+    sh->beat = s.beat;
     sh->tag = from ? from : *(volatile unsigned *)&s.sc->res_tag;
   }
   __syncthreads();

@@ -60,6 +60,7 @@ struct ResSys {
   int max_iter, eliminate;
   Scratch *sc;
   uint4 *xbuf;
+  unsigned *beat;  // counts on while the solve proceeds (null: nobody looks)
 };
 
 // CTAs of the resident solve that fit on the device at once, and how many of them in
@@ -78,9 +79,10 @@ int cgr_launch_sys(const ResSys &s, int rows, int clustered, cudaStream_t stream
 // Batched: CTA c runs jobs[job_start[c] .. job_start[c+1]) in order, then
 // single-CTA jobs from `singles` (*taken zero at the launch).  Every CTA's list
 // keeps the domains in one common order, so that no two groups wait for each
-// other.  CgJob::flags bits 4 and up: rows per thread.
+// other.  CgJob::flags bits 4 and up: rows per thread.  bsync: the batch's counters
+// (taken zero at the launch, and every domain's Scratch::res_arrived).
 int cgr_launch_batch(const View *views2, const int *job_start, const CgJob *jobs, const CgJob *singles,
-                     int nsingles, int *taken, int nctas, int any_mixed, cudaStream_t stream);
+                     int nsingles, Scratch *bsync, int nctas, int any_mixed, cudaStream_t stream);
 
 }  // namespace frehd
 

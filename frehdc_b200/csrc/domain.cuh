@@ -98,6 +98,8 @@ struct Scratch {
   int n_done;                // batched solve over a tile list: domains whose solve ended
   int taken;                 // batched resident solve: single-CTA solves handed out
   unsigned res_tag;          // resident solve: the last tag its exchange entries carry
+  unsigned res_arrived;      // batched resident solve: CTAs of this step's solve that are there
+  unsigned beat;             // (a batch's) signs of life of its resident solves
   int pad2;
 };
 

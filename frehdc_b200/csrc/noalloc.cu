@@ -311,7 +311,7 @@ extern "C" int frehd_cg_solve_noalloc(int nx, int ny, const double *Ct, const do
   if (rows) {
     ResSys sys{nx, ny, nx, 0, Ct, Gx, Gy, b, x0_from_x ? x : nullptr, x, eps, max_iter, 1,
                reinterpret_cast<Scratch *>(s->scratch),
-               reinterpret_cast<uint4 *>(s->scratch + kHeaderDoubles + kPartialDoubles)};
+               reinterpret_cast<uint4 *>(s->scratch + kHeaderDoubles + kPartialDoubles), nullptr};
     if ((rc = cgr_launch_sys(sys, rows, s->res_clustered, st)) != FREHD_OK) return rc;
     return read_result(s, st, iters, rel_residual);
   }

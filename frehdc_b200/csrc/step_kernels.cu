@@ -1230,6 +1230,7 @@ __global__ void k_finish_batch(const View *views2, const FinishJob *jobs, Scratc
   stage_view(views2, f.d, &sv, &s_cur, threadIdx.x, blockDim.x);
   const bool ran = finish_block(sv, f.nblocks_vel, f.out);
   if (ran && threadIdx.x == 0) sv.sc->cur = s_cur ^ 1;
+  if (threadIdx.x == 0) sv.sc->res_arrived = 0;
   // the batch's owner sees a failed domain (CFL > 20, a wait that gave up) after
   // this step without reading the domain's statistics
   if (threadIdx.x == 0) *(volatile int *)f.status = *(volatile int *)&sv.sc->status;
