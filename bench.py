@@ -639,11 +639,11 @@ def measure_batched(args, ws, rank, dev, n_mix, smin, smax, scalars, total_steps
         g.set_profiling(False)
     # packing of the solve and inner tolerance from the autotuner, tuned on rank
     # 0's share and used by every rank (a given cells_per_cta selects CTA groups)
+    from frehdc_b200 import autotune
     tuning = None
     cpc, eps_inner = args.cells_per_cta, args.eps_inner
     packing = "cta_groups" if cpc > 0 else "tile_list"
     if cpc <= 0:
-        from frehdc_b200 import autotune
         if rank == 0:
             tuning = autotune.tune(decks, budget, prec, device=dev)
         tuning = shard.broadcast(tuning, ws)
@@ -655,7 +655,10 @@ def measure_batched(args, ws, rank, dev, n_mix, smin, smax, scalars, total_steps
         tpb = args.tiles_per_block
     if eps_inner is None:
         eps_inner = 1e-4
-    pk = native.BATCH_TILE_LIST if packing == "tile_list" else native.BATCH_CTA_GROUPS
+    pk = autotune.PACKINGS[packing]
+    # on-chip and streaming solves are launches of their own
+    on_chip = {autotune.fits_on_chip(sp.nx, sp.ny) for sp in specs}
+    launches = 6 if packing == "cta_groups" and len(on_chip) == 2 else 5
     doms = [native.domain_from_deck(dk, device=dev, precision=prec, eps_inner=eps_inner)
             for dk in decks]
     b = native.Batch(budget, cpc if cpc > 0 else 1.0, dev)
@@ -701,7 +704,7 @@ def measure_batched(args, ws, rank, dev, n_mix, smin, smax, scalars, total_steps
         # solve's sums added in the other packing's order (rounding only), and
         # with the CG tolerance tightened tenfold (another solution that meets
         # the same residual bound); wet/dry branches amplify either difference
-        other = native.BATCH_CTA_GROUPS if pk == native.BATCH_TILE_LIST else native.BATCH_TILE_LIST
+        other = native.BATCH_CTA_GROUPS_STREAMED if pk == native.BATCH_TILE_LIST else native.BATCH_TILE_LIST
         names = ["surf", "uuXP", "vvYP"]
         ref_state = [(r.download(names), r.stats()["volume"]) for r in ref]
 
@@ -753,7 +756,7 @@ def measure_batched(args, ws, rank, dev, n_mix, smin, smax, scalars, total_steps
                                   "tide 0.1-0.5 m, n 0.02-0.04, 4x4 subgrid, "
                                   f"{scalars} scalar(s)",
                       "cells": int(total_cells), "packing": packing,
-                      "cells_per_cta": cpc if packing == "cta_groups" else None,
+                      "cells_per_cta": cpc if packing != "tile_list" else None,
                       "eps_inner": eps_inner if precision == "mixed" else None,
                       "stencil_tiles_per_block": tpb,
                       "sharding": "by cell count over ranks" if ws > 1 else None,
@@ -762,7 +765,7 @@ def measure_batched(args, ws, rank, dev, n_mix, smin, smax, scalars, total_steps
                                    "note": "each domain stepped alone in FP64, device time of "
                                            "its kernels summed over the mix"},
            "batch": parts[0]["info"] if ws == 1 else [p["info"] for p in parts],
-           "gpu_launches_timed": 5 * K, "clocks": parts[0]["clocks"]}
+           "gpu_launches_timed": launches * K, "clocks": parts[0]["clocks"]}
     rec["speedup_vs_plain_form"] = rec["value"] / rec["plain_form_same_mix"]["value"]
     if ws > 1:
         rec["per_rank"] = [{"domains": p["domains"], "cells": p["cells"],
@@ -801,7 +804,7 @@ def measure_served(args, ws, rank, dev, n_stream, n_req, smin, smax, steps_lo, s
     import numpy as np
 
     from frehdc_b200 import deck as D
-    from frehdc_b200 import native, serve, shard
+    from frehdc_b200 import autotune, native, serve, shard
     rng = np.random.default_rng(5)
     specs = mix_specs(n_stream, 91, smin, smax, 10, (1, scalars_max))[:n_req]
     steps = rng.integers(steps_lo, steps_hi + 1, size=n_stream)[:n_req]
@@ -817,6 +820,9 @@ def measure_served(args, ws, rank, dev, n_stream, n_req, smin, smax, steps_lo, s
     check = [i for i in mine if i % check_every == 0] if precision == "mixed" else []
     served_state = {}
 
+    # on-chip solves win as long as every domain fits on chip (frehd_batch_set_resident)
+    resident = all(autotune.fits_on_chip(sp.nx, sp.ny) for sp in specs)
+
     def build(req):
         return native.domain_from_deck(req.deck, device=dev, precision=prec, eps_inner=eps_inner)
 
@@ -829,7 +835,7 @@ def measure_served(args, ws, rank, dev, n_stream, n_req, smin, smax, steps_lo, s
         torch.distributed.barrier()
     with ClockSampler(dev) as clk:
         res = serve.serve(reqs, args.budget_gb << 30, cells_per_cta, device=dev, build=build,
-                          on_done=done)
+                          on_done=done, resident=resident)
     per = []
     for i in check:
         g = native.domain_from_deck(decks[i], device=dev)
@@ -848,6 +854,7 @@ def measure_served(args, ws, rank, dev, n_stream, n_req, smin, smax, steps_lo, s
                                   f"(square or 1:4), steps {steps_lo}-{steps_hi}, "
                                   f"1-{scalars_max} scalars, {precision}",
                       "requests": n_req, "cells_per_cta": cells_per_cta,
+                      "solves": "on chip" if resident else "streamed",
                       "eps_inner": eps_inner if precision == "mixed" else None,
                       "sharding": "least assigned work, arrival order" if ws > 1 else None,
                       "deck_gen_s": round(max(p["gen_s"] for p in parts), 1)},

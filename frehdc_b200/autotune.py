@@ -1,7 +1,8 @@
 """Autotuner of the batched form: picks the packing of the batched CG -- the
 tile list over all CTAs, or CTA groups with a granularity cells_per_cta (how
 many cells of a domain one CTA of its CG carries, hence how many CTAs each
-domain's solve gets and how the single-CTA domains are packed) -- and, for the
+domain's solve gets and how the single-CTA domains are packed), with the domains
+that fit on chip solved there or all of them streamed -- and, for the
 mixed-precision form, the inner FP32 tolerance, by timing a few batch steps of
 the actual mix with each candidate; then, at the chosen solve, the number of
 32 x 8 stencil tiles each block of the batched stencil kernels runs.
@@ -23,13 +24,22 @@ CELLS_PER_CTA = (8192.0, 16384.0, 32768.0, 65536.0, 131072.0, 196608.0, 229376.0
 EPS_INNER = (1e-4, 1e-5, 1e-6)
 TILES_PER_BLOCK = (1, 2, 4, 8)
 CTX, CTY = 128, 16   # CG tile of k_cg1
+PACKINGS = {"tile_list": native.BATCH_TILE_LIST, "cta_groups": native.BATCH_CTA_GROUPS,
+            "cta_groups_streamed": native.BATCH_CTA_GROUPS_STREAMED}
+
+
+def fits_on_chip(nx: int, ny: int, ctas: int = 148) -> bool:
+    """Whether a domain's solver state fits on chip: one CTA per tile of 64 x 64 cells
+    at most (csrc/cg_res.h, res_rows)."""
+    return ((nx + 63) // 64) * ((ny + 63) // 64) <= ctas
 
 
 def ctas_needed(sizes, cells_per_cta: float, capacity: int = 148) -> int:
     """CTAs of the batched CG for domains of these (nx, ny): each domain's
     group is ceil(cells / cells_per_cta) CTAs (at least 1, at most its tile
     count), multi-CTA groups get CTAs of their own and the single-CTA domains
-    share the rest (batch.cu, group_size / ctas_needed)."""
+    share the rest (batch.cu, group_size / ctas_needed).  Admission counts the
+    domains solved on chip the same way, although their solves share CTAs."""
     dedicated, singles = 0, 0
     for nx, ny in sizes:
         ntiles = ((nx + CTX - 1) // CTX) * ((ny + CTY - 1) // CTY)
@@ -81,7 +91,8 @@ def tune(decks, budget: int, precision: int = native.PRECISION_FP64, steps: int 
          device: int = 0) -> dict:
     """The fastest (packing, cells_per_cta, eps_inner) on this mix, then the
     fastest stencil tiles per block with it, and every timing.  The tile-list
-    packing takes any mix; CTA-group granularities whose CG would need more
+    packing takes any mix; CTA groups are tried with and without on-chip solves
+    (if any domain fits); granularities whose CG would need more
     co-resident CTAs than the device holds are skipped before any domain is
     built.  The domains are built once and stepped by every candidate in turn."""
     eps_list = eps_candidates if precision == native.PRECISION_MIXED else (1e-5,)
@@ -89,7 +100,9 @@ def tune(decks, budget: int, precision: int = native.PRECISION_FP64, steps: int 
     sizes = [(dk.nx, dk.ny) for dk in decks]
     fits = [c for c in cells_candidates if ctas_needed(sizes, c, capacity) <= capacity]
     cands = [("tile_list", 0.0)] + [("cta_groups", c) for c in fits]
-    packings = {"tile_list": native.BATCH_TILE_LIST, "cta_groups": native.BATCH_CTA_GROUPS}
+    if any(fits_on_chip(nx, ny) for nx, ny in sizes):
+        cands += [("cta_groups_streamed", c) for c in fits]
+    packings = PACKINGS
     results = []
     doms = [native.domain_from_deck(dk, device=device) for dk in decks]
     try:

@@ -116,6 +116,7 @@ struct frehd_batch {
   int nrsingles = 0, nrctas = 0, any_rmixed = 0;
   // tile-list packing
   int packing = FREHD_BATCH_CTA_GROUPS;
+  int resident = 1;  // small domains solve on chip (CTA groups; frehd_batch_set_resident)
   int tiles_per_block = kTilesPerBlock;
   DevArray<BDom> bdoms;
   DevArray<BTile> btiles;
@@ -151,9 +152,16 @@ int group_size(const frehd_batch *b, const frehd_domain *d) {
 // Rows per thread of domain d's resident solve in this batch (0: it streams).
 // cells_per_cta asks for tiles of that many cells (up to the largest tile): few
 // large tiles keep more domains in flight, many small ones shorten one solve.  By
-// the domain's size alone, so that its result is the same in any mix.
+// the domain's size and the batch's settings alone, so that its result is the same in
+// any mix.  The setting is the caller's because no such rule decides it: as long as
+// every domain fits on chip the resident solves win by far (24 basins of 64-512 cells
+// a side, mixed: 1.8 ms a step against 4.2 at 65536 cells per CTA and 11.9 at 262144;
+// 100 basins 6.2 against 9.3 and 15.0), but beside domains that stream they lose,
+// since the two launches follow each other and the longest group bounds the streaming
+// one whatever runs with it (256 basins of 64-1024 at 393216: 65.9 ms against 50.4; 64
+// of them at 262144: 22.8 against 18.6).
 int resident_rows(const frehd_batch *b, const frehd_domain *d) {
-  if (!d->res_rows) return 0;
+  if (!b->resident || !d->res_rows) return 0;
   for (int KR = d->res_rows; KR < kResMaxKR; KR *= 2)
     if (kResTW * res_th(KR) >= b->cells_per_cta) return KR;
   return kResMaxKR;
@@ -664,6 +672,15 @@ extern "C" int frehd_batch_set_cg_packing(frehd_batch *b, int packing) {
     }
   }
   b->packing = packing;
+  b->dirty = true;
+  return FREHD_OK;
+}
+
+extern "C" int frehd_batch_set_resident(frehd_batch *b, int on) {
+  if (!b) return fail(FREHD_ERR_INVALID, "null batch");
+  BATCH_TRY(cudaSetDevice(b->device));
+  BATCH_TRY(cudaStreamSynchronize(b->stream));  // queued steps use the current tables
+  b->resident = on ? 1 : 0;
   b->dirty = true;
   return FREHD_OK;
 }

@@ -231,6 +231,15 @@ extern "C" int frehd_server_create(int device, long long hbm_budget_bytes, doubl
   return FREHD_OK;
 }
 
+extern "C" int frehd_server_set_resident(frehd_server *s, int on) {
+  clear_error();
+  if (!s) return fail(FREHD_ERR_INVALID, "null server");
+  std::lock_guard<std::mutex> lk(s->mu);  // with no request held the thread waits for one
+  if (!s->waiting.empty() || !s->active.empty())
+    return fail(FREHD_ERR_STATE, "the server holds requests");
+  return frehd_batch_set_resident(s->batch, on);
+}
+
 extern "C" int frehd_server_submit(frehd_server *s, frehd_domain *d, int t0, int nsteps,
                                    long long *ticket) {
   clear_error();

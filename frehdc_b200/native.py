@@ -147,7 +147,7 @@ CG_SINGLE_SWEEP, CG_TWO_PHASE = 0, 1
 DECOUPLED_AS_ASSEMBLED, DECOUPLED_ELIMINATED = 0, 1
 PRECISION_FP64, PRECISION_MIXED = 0, 1
 SERIES_TIDE, SERIES_INFLOW, SERIES_WIND_SPEED, SERIES_WIND_DIR = 0, 1, 2, 3
-BATCH_TILE_LIST, BATCH_CTA_GROUPS = 0, 1
+BATCH_TILE_LIST, BATCH_CTA_GROUPS, BATCH_CTA_GROUPS_STREAMED = 0, 1, 2
 STATUS = {0: "ok", 1: "invalid", 2: "unsupported", 3: "cuda", 4: "nomem", 5: "cg_noconverge",
           6: "cfl", 7: "timeout", 8: "state"}
 
@@ -456,6 +456,8 @@ def _declare_batch(L: C.CDLL) -> None:
     L.frehd_batch_stream.argtypes = [_vp, C.POINTER(_vp)]
     L.frehd_batch_set_graph.argtypes = [_vp, C.c_int]
     L.frehd_batch_set_cg_packing.argtypes = [_vp, C.c_int]
+    L.frehd_batch_set_resident.argtypes = [_vp, C.c_int]
+    L.frehd_server_set_resident.argtypes = [_vp, C.c_int]
     L.frehd_batch_set_stencil_tiles.argtypes = [_vp, C.c_int]
     L.frehd_server_create.argtypes = [C.c_int, C.c_longlong, C.c_double, C.POINTER(_vp)]
     L.frehd_server_submit.argtypes = [_vp, _vp, C.c_int, C.c_int, C.POINTER(C.c_longlong)]
@@ -552,8 +554,12 @@ class Batch:
         check(lib().frehd_batch_set_graph(self.h, int(on)), "frehd_batch_set_graph")
 
     def set_cg_packing(self, packing: int):
-        """BATCH_CTA_GROUPS (default) or BATCH_TILE_LIST (frehd_batch_set_cg_packing)."""
-        check(lib().frehd_batch_set_cg_packing(self.h, int(packing)), "frehd_batch_set_cg_packing")
+        """BATCH_CTA_GROUPS (default), BATCH_CTA_GROUPS_STREAMED (the same without on-chip
+        solves) or BATCH_TILE_LIST (frehd_batch_set_cg_packing, frehd_batch_set_resident)."""
+        streamed = packing == BATCH_CTA_GROUPS_STREAMED
+        check(lib().frehd_batch_set_cg_packing(self.h, BATCH_CTA_GROUPS if streamed else int(packing)),
+              "frehd_batch_set_cg_packing")
+        check(lib().frehd_batch_set_resident(self.h, 0 if streamed else 1), "frehd_batch_set_resident")
 
     def set_stencil_tiles(self, tiles_per_block: int):
         """32 x 8 stencil tiles per block of the batched stencil kernels, 1..8
@@ -587,6 +593,10 @@ class Server:
               "frehd_server_create")
         self.h = h
         self.held: dict[int, "Domain"] = {}
+
+    def set_resident(self, on: bool):
+        """On-chip solves of the domains that fit (frehd_server_set_resident)."""
+        check(lib().frehd_server_set_resident(self.h, int(on)), "frehd_server_set_resident")
 
     def submit(self, dom: "Domain", nsteps: int, t0: int = 1) -> int:
         t = C.c_longlong()

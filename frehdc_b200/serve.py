@@ -49,19 +49,23 @@ def poisson_arrivals(n: int, rate: float, seed: int) -> np.ndarray:
 
 
 def serve(requests: list[Request], budget_bytes: int, cells_per_cta: float, device: int = 0,
-          build=None, on_done=None) -> dict:
+          build=None, on_done=None, resident: bool = True) -> dict:
     """Serve the requests; returns latency percentiles (and every request's
     latency, in completion order) and throughput.
 
     build(req) -> native.Domain sets up a request's domain (default: from its
     deck, fine geometry); on_done(req) is called right after the request
-    completes (the domain's state can be downloaded there)."""
+    completes (the domain's state can be downloaded there).  resident=False: every
+    solve streams (frehd_server_set_resident: faster where large domains are among
+    the requests)."""
     import threading
 
     if build is None:
         def build(req):
             return native.domain_from_deck(req.deck, device=device, geometry="fine")
     server = native.Server(budget_bytes, cells_per_cta, device)
+    if not resident:
+        server.set_resident(False)
     order = sorted(requests, key=lambda r: r.arrival)
     by_ticket: dict[int, Request] = {}
     lock = threading.Lock()

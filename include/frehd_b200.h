@@ -469,6 +469,13 @@ int frehd_batch_set_graph(frehd_batch *b, int on);
  * domains do not fit the CTA groups (the packing then stays the tile list). */
 enum { FREHD_BATCH_TILE_LIST = 0, FREHD_BATCH_CTA_GROUPS = 1 };
 int frehd_batch_set_cg_packing(frehd_batch *b, int packing);
+/* CTA groups: whether domains that fit on chip solve there (default 1) or stream like
+ * the larger ones (0).  On chip is faster by two to ten times while all domains of the
+ * batch fit.  In a mix with larger ones, whose launch follows, streaming all of them is
+ * faster (a quarter with 256 basins of 64 to 1024 cells a side): the autotuner tries
+ * both.  The two agree to the solver's rounding; in either a domain's result is the
+ * same in any mix. */
+int frehd_batch_set_resident(frehd_batch *b, int on);
 /* Stencil tiles (32 x 8 cells, consecutive along a row of one domain) each
  * block of the batched stencil kernels runs, 1..8 (default 4): more tiles per
  * block stage the domain's view fewer times, fewer give more blocks to spread
@@ -508,6 +515,9 @@ typedef struct frehd_server_info_t {
 
 int frehd_server_create(int device, long long hbm_budget_bytes, double cells_per_cta,
                         frehd_server **out);
+/* frehd_batch_set_resident for the server's batch; FREHD_ERR_STATE while it holds
+ * requests. */
+int frehd_server_set_resident(frehd_server *s, int on);
 int frehd_server_submit(frehd_server *s, frehd_domain *d, int t0, int nsteps, long long *ticket);
 /* Up to cap completed requests into out (*n of them); waits up to timeout_ms
  * for the first one when none is ready (0: return at once). */
