@@ -76,6 +76,9 @@ static __device__ __forceinline__ bool grid_allreduce(double (&v)[NV], Scratch *
   if (s_last) {
     // every partial is visible: sum them in a fixed order, publish, release
     __threadfence();
+    // (one thread looks whether a block has given up: read by each, the status could
+    // part the threads of a block before its next barrier)
+    const int status = threadIdx.x == 0 ? *(volatile int *)&sc->status : 0;
     double a[NV];
 #pragma unroll
     for (int m = 0; m < NV; ++m) a[m] = 0;
@@ -97,6 +100,7 @@ static __device__ __forceinline__ bool grid_allreduce(double (&v)[NV], Scratch *
         for (int q = 0; q < NWARP; ++q) t += sh[m][q];
         totals[m] = t;
       }
+      if (status == FREHD_ERR_TIMEOUT) s_ok = 0;
       *(volatile unsigned *)&sc->bar_count = 0;
       __threadfence();
       atomicAdd(&sc->bar_gen, 1u);
@@ -105,7 +109,14 @@ static __device__ __forceinline__ bool grid_allreduce(double (&v)[NV], Scratch *
     volatile unsigned *gen = &sc->bar_gen;
     const unsigned long long lim = sc->wait_limit_ns ? sc->wait_limit_ns : kBarrierTimeoutNs;
     const unsigned long long t0 = gtimer_ns();
-    while (*gen == my_gen) {
+    // (the status comes with the generation: on its own it would cost a round trip more)
+    for (;;) {
+      const unsigned now = *gen;
+      const int status = *(volatile int *)&sc->status;
+      if (now != my_gen) {
+        if (status == FREHD_ERR_TIMEOUT) s_ok = 0;
+        break;
+      }
       if (gtimer_ns() - t0 > lim) {
         set_status(sc, FREHD_ERR_TIMEOUT);
         s_ok = 0;
@@ -116,7 +127,7 @@ static __device__ __forceinline__ bool grid_allreduce(double (&v)[NV], Scratch *
     __threadfence();
   }
   __syncthreads();
-  if (!s_ok || *(volatile int *)&sc->status == FREHD_ERR_TIMEOUT) return false;
+  if (!s_ok) return false;
 #pragma unroll
   for (int m = 0; m < NV; ++m) v[m] = ld(totals, m);
   return true;
