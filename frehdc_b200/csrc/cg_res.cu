@@ -57,27 +57,27 @@ __device__ __forceinline__ bool res_arrive(Scratch *sc, unsigned nb, unsigned *b
 // The two solves as functions of their own: in one kernel with each other or with
 // other tile heights they must not share a register allocation (the inlined FP32
 // sweeps of 64 x 64 tiles spilled 2.6 KB).
-template <int KR>
+template <int KR, bool kBatch>
 __device__ __noinline__ ResEnd res_job_mixed(const ResSys *sp, double eps_inner, unsigned rank, unsigned nb,
                                           unsigned csize) {
   extern __shared__ __align__(16) double res_sm[];
   __shared__ ResShared sh;
   const ResSys s = *sp;
-  return res_mixed<KR>(s, eps_inner, rank, nb, csize, res_sm, &sh);
+  return res_mixed<KR, kBatch>(s, eps_inner, rank, nb, csize, res_sm, &sh);
 }
-template <int KR>
+template <int KR, bool kBatch>
 __device__ __noinline__ bool res_job_fp64(const ResSys *sp, unsigned rank, unsigned nb, unsigned csize,
                                           unsigned from) {
   extern __shared__ __align__(16) double res_sm[];
   __shared__ ResShared sh;
   const ResSys s = *sp;
-  return res_fp64<KR>(s, rank, nb, csize, from, res_sm, &sh);
+  return res_fp64<KR, kBatch>(s, rank, nb, csize, from, res_sm, &sh);
 }
 
 // The domain's solve in its configured precision by nb CTAs (in clusters of csize); sp
 // in shared memory.  kAlone: the FP64 solve is the kernel's only one (inlined: 4.56 us
 // per iteration at 512 x 512 against 5.39).
-template <int KR, bool kMix, bool kAlone = false>
+template <int KR, bool kMix, bool kAlone, bool kBatch>
 __device__ __forceinline__ void res_solve(const ResSys *sp, int mixed, double eps_inner, unsigned rank, unsigned nb,
                                           unsigned csize) {
   if (test_skip_barrier(sp->sc, rank)) {  // a lone CTA has no partner whose wait could run out
@@ -85,18 +85,18 @@ __device__ __forceinline__ void res_solve(const ResSys *sp, int mixed, double ep
     return;
   }
   if (kMix && mixed) {
-    const ResEnd end = res_job_mixed<KR>(sp, eps_inner, rank, nb, csize);
+    const ResEnd end = res_job_mixed<KR, kBatch>(sp, eps_inner, rank, nb, csize);
     if (end.code != 2) return;
-    if (res_job_fp64<KR>(sp, rank, nb, csize, end.tag) && rank == 0 && threadIdx.x == 0) sp->sc->cg_fallback = 2;
+    if (res_job_fp64<KR, kBatch>(sp, rank, nb, csize, end.tag) && rank == 0 && threadIdx.x == 0) sp->sc->cg_fallback = 2;
     return;
   }
   if (kAlone) {
     extern __shared__ __align__(16) double res_sm[];
     __shared__ ResShared sh;
     const ResSys s = *sp;
-    res_fp64<KR>(s, rank, nb, csize, 0, res_sm, &sh);
+    res_fp64<KR, kBatch>(s, rank, nb, csize, 0, res_sm, &sh);
   } else {
-    res_job_fp64<KR>(sp, rank, nb, csize, 0);
+    res_job_fp64<KR, kBatch>(sp, rank, nb, csize, 0);
   }
 }
 
@@ -135,7 +135,7 @@ __device__ __forceinline__ void res_kernel(Scratch *sc, int mixed, double eps_in
     if (s_run) fill(&s);
   }
   __syncthreads();
-  if (s_run) res_solve<KR, kMix, !kMix>(&s, mixed, eps_inner, blockIdx.x, nb, csize);
+  if (s_run) res_solve<KR, kMix, !kMix, false>(&s, mixed, eps_inner, blockIdx.x, nb, csize);
   // no store into this CTA's shared memory is on its way any more
   if (csize > 1) res_cluster_sync();
 }
@@ -184,9 +184,9 @@ __global__ void __launch_bounds__(kResThreads, 1)
     if (!s_run) continue;
     // a solve that gave up has marked its own domain; the CTA goes on with the next
     switch (jb.flags >> 4) {
-      case 1: res_solve<1, kMix>(&s_sys, s_mixed, s_eps, jb.rank, jb.nb, 1); break;
-      case 2: res_solve<2, kMix>(&s_sys, s_mixed, s_eps, jb.rank, jb.nb, 1); break;
-      default: res_solve<4, kMix>(&s_sys, s_mixed, s_eps, jb.rank, jb.nb, 1); break;
+      case 1: res_solve<1, kMix, false, true>(&s_sys, s_mixed, s_eps, jb.rank, jb.nb, 1); break;
+      case 2: res_solve<2, kMix, false, true>(&s_sys, s_mixed, s_eps, jb.rank, jb.nb, 1); break;
+      default: res_solve<4, kMix, false, true>(&s_sys, s_mixed, s_eps, jb.rank, jb.nb, 1); break;
     }
     if (threadIdx.x == 0) atomicAdd(&bsync->beat, 1u);
   }

@@ -49,8 +49,9 @@ namespace frehd {
 
 struct ResShared {
   double tot[kResSlot];
+  double scale, inv_gamma;  // 1 / (scale gamma) of the last sweep (res_keep)
   unsigned tag;    // the tag the solve starts from
-  unsigned *beat;  // ResSys::beat
+  unsigned *beat;  // ResSys::beat (batched solves)
   int ok;
 };
 
@@ -279,7 +280,6 @@ __device__ __forceinline__ bool res_allreduce(double (&v)[kResSums], const ResCt
     if (lane == 0) sh->tot[wid] = t;
   } else {
     meanwhile();
-    if (threadIdx.x == kResThreads - 1 && (c.tag & (kResBeat - 1)) == 0 && sh->beat) atomicAdd(sh->beat, 1u);
   }
   __syncthreads();
 #pragma unroll
@@ -834,10 +834,29 @@ __device__ __forceinline__ void res_leave(const ResSys &s, const ResCtx &c) {
   atomicMax(&s.sc->res_tag, c.tag);
 }
 
+// What a warp without a sum keeps of a sweep while the sums travel: the reciprocal of
+// gamma = (r~, r~), scaled by a power of two where 1 / gamma would not be a normal
+// number; in a batch also the sign of life.  (The division in the iteration's chain
+// cost 2 us of a 59 us solve at 128 x 128 and 20 of 285 at 512 x 512.)
+template <bool kBatch>
+__device__ __forceinline__ void res_keep(const ResCtx &c, double gamma) {
+  if (threadIdx.x >> 5 != kResSums) return;
+  const double scale = gamma < 0x1p-512 ? 0x1p600 : gamma > 0x1p512 ? 0x1p-600 : 1.0;
+  c.sh->scale = scale;
+  c.sh->inv_gamma = 1.0 / (gamma * scale);
+  if (kBatch && (c.tag & (kResBeat - 1)) == 0 && (threadIdx.x & 31) == 0) atomicAdd(c.sh->beat, 1u);
+}
+
+// beta = gamma / (the last sweep's gamma).
+__device__ __forceinline__ double res_beta(double gamma, const ResShared *sh) {
+  return gamma * sh->scale * sh->inv_gamma;
+}
+
 // FP64 solve by nb CTAs, of which this one is number `rank` = its tile number.
-// sm: res_smem(KR) bytes of shared memory.  from: see res_enter.  False after an error
+// sm: res_smem(KR) bytes of shared memory.  from: see res_enter.  kBatch: other solves
+// wait for this one's signs of life (s.beat).  False after an error
 // (status set).
-template <int KR>
+template <int KR, bool kBatch>
 __device__ __forceinline__ bool res_fp64(const ResSys &s, unsigned rank, unsigned nb, unsigned csize, unsigned from,
                                          double *sm, ResShared *sh) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -909,7 +928,7 @@ __device__ __forceinline__ bool res_fp64(const ResSys &s, unsigned rank, unsigne
     red[3] = first[1];
     ++c.tag;
     if (!(ok = res_allreduce<4>(red, c, [] {}))) break;
-    double gamma = red[0], gamma_old = 1.0, delta = red[3], e1 = 0.0, e2 = 0.0, e3 = 0.0;
+    double gamma = red[0], delta = red[3], e1 = 0.0, e2 = 0.0, e3 = 0.0;
     rr = red[1];
     bnorm = sqrt(red[2]);
     limit = res_limit(bnorm, s.eps);
@@ -918,7 +937,7 @@ __device__ __forceinline__ bool res_fp64(const ResSys &s, unsigned rank, unsigne
     bool stalled = false;
     it = 0;
     while (!(rr <= limit) && it < s.max_iter) {
-      const double beta = it == 0 ? 0.0 : gamma / gamma_old;
+      const double beta = it == 0 ? 0.0 : res_beta(gamma, sh);
       const double alpha = gamma / (delta + beta * (e1 + e2) + beta * beta * e3);
       ++it;
       ++c.tag;
@@ -955,11 +974,11 @@ __device__ __forceinline__ bool res_fp64(const ResSys &s, unsigned rank, unsigne
         }
       }
       ok = res_allreduce<6>(red, c, [&] {
+        res_keep<kBatch>(c, gamma);
         res_ring_take<double, KR>(c, t);
         ring_stencil();
       });
       if (!ok) break;
-      gamma_old = gamma;
       gamma = red[0];
       delta = red[1];
       e1 = red[2];
@@ -1011,7 +1030,7 @@ __device__ __forceinline__ bool res_fp64(const ResSys &s, unsigned rank, unsigne
 // refinement (cg1_mixed in cg1.cu, same steps, same stopping rules).  x lives in
 // registers; between two inner solves it goes through global memory, where the
 // next residual reads its neighbours.
-template <int KR>
+template <int KR, bool kBatch>
 __device__ __forceinline__ ResEnd res_mixed(const ResSys &s, double eps_inner, unsigned rank, unsigned nb, unsigned csize,
                                          double *sm, ResShared *sh) {
   constexpr int kArr = res_arr(KR);
@@ -1075,23 +1094,25 @@ __device__ __forceinline__ ResEnd res_mixed(const ResSys &s, double eps_inner, u
     if (outer > 0 && rr > 1e-2 * rr_prev) break;  // no tenfold gain: FP64 takes over
     rr_prev = rr;
     // A~ d~ = r~ until (r~, r~) fell by eps_inner^2
-    double gamma = red[0], gamma_old = 1.0, delta = red[3], e1 = 0.0, e2 = 0.0, e3 = 0.0;
+    double gamma = red[0], delta = red[3], e1 = 0.0, e2 = 0.0, e3 = 0.0;
     const double stop = eps_inner * eps_inner * gamma;
 #pragma unroll
     for (int k = 0; k < KR; ++k) t.x[k][0] = t.x[k][1] = 0.0f;
     int it = 0;
     bool ok = true;
     while (gamma > stop && it < s.max_iter) {
-      const double beta = it == 0 ? 0.0 : gamma / gamma_old;
+      const double beta = it == 0 ? 0.0 : res_beta(gamma, sh);
       const double alpha = gamma / (delta + beta * (e1 + e2) + beta * beta * e3);
       const int cur = it & 1;
       ++it;
       ++c.tag;
       res_sweep32<KR>(c, t, P + 2 * cur * kArr, R + 2 * cur * kArr, P + 2 * (cur ^ 1) * kArr,
                       R + 2 * (cur ^ 1) * kArr, (float)alpha, (float)beta, p2, red);
-      ok = res_allreduce<5>(red, c, [&] { res_ring_take<float, KR>(c, t); });
+      ok = res_allreduce<5>(red, c, [&] {
+        res_keep<kBatch>(c, gamma);
+        res_ring_take<float, KR>(c, t);
+      });
       if (!ok) break;
-      gamma_old = gamma;
       gamma = red[0];
       delta = red[1];
       e1 = red[2];
