@@ -23,7 +23,8 @@ and the other forms of the metric, each a sub-record with its own config:
                refinement): device rate, and eta/u/v/scalar/volume errors against
                the FP64 run after 1000 steps
   batched      256 seeded basins, sides 64-1024, 2 scalars, mixed precision, one
-               batch (five launches per step, graph-replayed), autotuned packing:
+               batch (five launches per step, six where on-chip and streaming solves
+               mix; graph-replayed), autotuned packing:
                rate, the same mix stepped one domain at a time in FP64, the
                speed-up, and errors against FP64 after 500 steps
   served       the head of a 2000-request stream (Poisson arrivals 50/s, sides
@@ -456,6 +457,8 @@ def report(args, kt, st, iters, t_max, value, ws, n, spec, gen_s, e2e, clk, sub=
     cg_cell = cg_bytes_per_cell(iters, fp64)
     cg_bytes = N * cg_cell
     achieved = cg_bytes / (cg_launch_ms / 1e3) / 1e9
+    from frehdc_b200 import autotune
+    on_chip = args.cg_schedule == "single_sweep" and autotune.fits_on_chip(n, n)
     kname = {"single_sweep": "k_cg1 (persistent single-sweep Jacobi-PCG, one launch per step)",
              "two_phase": "k_cg (persistent two-phase Jacobi-PCG, one launch per step)"}
     roof = {"kernel": kname[args.cg_schedule], "bound": "hbm",
@@ -466,6 +469,9 @@ def report(args, kt, st, iters, t_max, value, ws, n, spec, gen_s, e2e, clk, sub=
                             "refinement sweeps not counted)"),
             "bytes_per_cell": cg_cell,
             "cg_iters_per_step": iters, "launch_ms": cg_launch_ms}
+    if on_chip:  # the solver state stays on chip: the byte model describes no traffic of it
+        roof.update(kernel="k_cgr (Jacobi-PCG with its state on chip, one launch per step)",
+                    bound="latency", achieved=None, frac=None, bytes_model=None, bytes_per_cell=None)
     # DRAM traffic of one launch from the committed ncu summary (scaled from a
     # smaller capture; it describes the 4096^2 single-sweep solve only)
     prof = os.path.join(REPO, "profiles", "k_cg1_2048x2048_fp64.md")

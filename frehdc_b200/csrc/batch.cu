@@ -3,22 +3,24 @@
 // Domains are set up one by one with the single-domain calls (create, geometry,
 // tide, init), then admitted into a batch, which owns their stepping until they
 // are released.  One batch step advances every admitted domain by one time step
-// with five launches in total, whatever the number of domains:
+// with five to seven launches in total, whatever the number of domains:
 //   k_explicit_batch, k_update_geo_batch, k_update_vel_batch   one block per
-//       (domain, 32 x 8 tile) entry of a tile table over all domains
-//   the solve, one cooperative launch over all co-resident CTAs, in one of two
+//       (domain, 32 x 8 tile) entry of a tile table over all domains (domains with
+//       TVD advection have a velocity kernel of their own)
+//   the solve, cooperative launches over all co-resident CTAs, in one of two
 //       packings (frehd_batch_set_cg_packing):
 //     k_cg1_batch (FREHD_BATCH_CTA_GROUPS, the default): each domain solved by a group of
 //       CTAs whose size depends on the domain's own cell count only (multi-CTA
 //       groups on CTAs of their own; single-CTA domains, longest first, taken
 //       one after another by whichever CTA is free).  Domains whose solver state
-//       fits on chip run in k_cgr_batch instead: each on as many CTAs as its tiles,
-//       the CTAs taking one domain after another in a fixed schedule
+//       fits on chip run in k_cgr_batch instead, a launch before: each on as many
+//       CTAs as its tiles, the CTAs taking one domain after another in a fixed
+//       schedule (unless frehd_batch_set_resident has them stream)
 //     k_cg1_tiles (FREHD_BATCH_TILE_LIST): the CG tiles of every domain form one
 //       list spread over all CTAs; each domain's sums are added in its own tile
 //       order, so its result depends neither on the mix nor on cells_per_cta
 //   k_finish_batch   one block per domain; flips the domain's ping-pong half
-// The five launches are captured once per batch composition into a CUDA graph
+// The launches are captured once per batch composition into a CUDA graph
 // and replayed every step.
 //
 // Admission is by device-memory footprint (a budget given at creation) and, in
@@ -481,7 +483,7 @@ extern "C" int frehd_domain_footprint(const frehd_config *cfg, int r, long long 
   b += 36 * 8 * tot;                // persistent, per-step and CG arrays
   b += tot;                         // rmv flags
   b += 4 * N + 8 * T;               // fix list, staging
-  b += cgr_exchange_bytes(g, res_rows(cfg->nx, cfg->ny, 148));  // the resident solve's exchange
+  b += cgr_exchange_bytes(g, res_rows(cfg->nx, cfg->ny, 148));  // the on-chip solve's exchange (a B200's SMs)
   b += 8 * std::max(nvel, 8LL * 148 + 8) + 4096;  // partials, scratch, maps
   b += 8 * N * (long long)r * r;    // fine bottoms
   b += (20 * 8 + 2 * 4) * tot;      // level-value cache of the fine geometry

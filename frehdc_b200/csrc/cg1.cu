@@ -527,7 +527,8 @@ static __device__ __forceinline__ bool cg1_fp64(const View &w, const Cg1Maps *__
     if (threadIdx.x == 0) s_fallback = 1;
   }  // attempt
 
-  // ---- x = x~ / sqrt|Ct| (each block its own tiles)
+  // ---- x = x~ / sqrt|Ct| (some tiles were last written by another block, every other
+  // sweep being in reverse: the reduction in between makes them visible)
   for (int tile = rank; tile < ti.ntiles; tile += nb) {
     int i0, j0;
     tile_origin(ti, tile, &i0, &j0);

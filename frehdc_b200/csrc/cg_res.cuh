@@ -12,17 +12,20 @@
 //   * the tile's outer second row and column of the new residual (what a
 //     neighbour tile cannot compute itself: it recomputes the first ring), and
 //   * the CTA's six partial sums, added in an order fixed by the ranks.
-// Both travel as 16-byte entries {low word, tag, high word, tag}: the tag is the
-// reduction's number, so an entry announces itself and neither a fence nor an
-// arrival counter stands between the writer's store and the reader's load.  The
+// Both travel as 16-byte entries {low word, tag, high word, tag}, the layout and the one
+// 16-byte access of NCCL's LL protocol: the tag is the reduction's number, so an entry
+// announces itself and neither a fence nor an arrival counter stands between the
+// writer's store and the reader's load.  (An entry orders itself only: where other
+// memory is to be read after a reduction, res_exchange fences.)  The
 // entries alternate between two buffers by tag parity; no CTA can write the
 // buffer of reduction t + 2 before every CTA has published t + 1, that is,
 // finished reading t.
 //
 // The CTAs of one solve form clusters: of all of them up to kResFlat, of res_group up
-// to kResClustered (more do not fit the device in clusters).  Inside a cluster an entry is stored straight into its reader's shared
-// memory, where polling costs nothing (through L2 every reader polls the line that
-// its writer is waiting to store: 2.4 us a reduction among 16 CTAs).  Only the
+// to kResClustered (more do not fit the device in clusters).  Inside a cluster an entry
+// is stored straight into its reader's shared memory, where polling costs nothing
+// (through L2 every reader polls the line that its writer is waiting to store: 2.4 us a
+// reduction among 16 CTAs).  Only the
 // groups' sums and the edges between clusters go through L2.  In a batch, whose CTAs
 // take one solve after another in ever new groups, all entries do; the sums are added
 // in the same order either way.
@@ -37,7 +40,16 @@
 // rounding.
 //
 // Tags only grow: a launch starts at Scratch::res_tag, and every CTA raises it
-// to the last tag it used, whether it ends well or after a wait that gave up.
+// to the last tag it used, whether it ends well or after a wait that gave up.  Near
+// their end a solve clears the entries and starts them again (res_enter).
+//
+// Rounding: A p by its recurrence and the scaling by sqrt|Ct| are as good as the stencil
+// on p and the unscaled system while a solve takes hundreds of iterations (the error
+// against 64-bit references is the same to two digits up to 300, and to 2000 at
+// tolerances above 1e-13).  Past that, where a tolerance asks for all the digits that a
+// condition number near 1e7 and more leaves, the solution attained is further off:
+// 2e-14 against 8e-15 after 1000 iterations, 2e-11 against 2e-13 after 7400 (couplings
+// over six decades); the scaling, which k_cg1 has too, is most of it.
 #ifndef FREHD_CG_RES_CUH
 #define FREHD_CG_RES_CUH
 
@@ -867,8 +879,9 @@ __device__ __forceinline__ bool res_fp64(const ResSys &s, unsigned rank, unsigne
   if (!res_enter(s, rank, nb, csize, KR, from, sm, sh, &c)) return false;
   ResTile<double, KR> t;
   double w[KR][2], as[KR][2];  // A~ r~, A~ p
-  // x~ and |Ct| of the tallest tile's cells lie in shared memory (its registers would
-  // spill), those of the others in registers
+  // x~ and |Ct| of the tallest tile's cells lie in shared memory, those of the others in
+  // registers.  128 a thread do not hold all of it even so: 708 bytes of spill loads a
+  // thread for the tallest tile, 308 with two rows and 88 with one, partly in the set-up
   constexpr bool kShared = KR == kResMaxKR;
   double D[kShared ? 1 : KR][2];
   double2 *const xs = reinterpret_cast<double2 *>(R + res_arr(KR)) + threadIdx.x, *const Ds = xs + KR * kResThreads;
@@ -956,7 +969,9 @@ __device__ __forceinline__ bool res_fp64(const ResSys &s, unsigned rank, unsigne
         s1 = w1 + beta * s1;
         t.r1 = t.r1 - alpha * s1;
         R[t.q1] = t.r1;
-      } __syncthreads(); res_publish<double, KR>(c, t, R);
+      }
+      __syncthreads();
+      res_publish<double, KR>(c, t, R);
       res_stencil<KR>(t, R, diag, w, red);
 #pragma unroll
       for (int k = 0; k < KR; ++k) {

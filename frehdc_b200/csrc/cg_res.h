@@ -15,9 +15,9 @@ constexpr int kResWarps = 16, kResThreads = 32 * kResWarps;
 constexpr int kResMinKR = 1, kResMaxKR = 4;  // rows per thread: tiles 64 x 16, 64 x 32, 64 x 64
 constexpr int kResSlot = 8;             // entries per CTA in the reduction buffer (six sums)
 constexpr int kResFlat = 16;            // CTAs whose sums are added in one go, and the largest cluster
-// With more CTAs: how many form a group, and a cluster.  Eight, while they fit the
-// device (clusters of eight leave 120 of the 148 SMs usable, of four 132).
 constexpr int kResMaxOuter = 8;         // refinements of one mixed-precision solve
+// With more CTAs than kResFlat: how many form a group, and a cluster.  Eight, while they
+// fit the device (clusters of eight leave 120 of the 148 SMs usable, of four 132).
 constexpr int kResMaxGroups = 32, kResEights = 112, kResClustered = 4 * kResMaxGroups;
 __host__ __device__ constexpr int res_group(int nb) { return nb <= kResEights ? 8 : 4; }
 __host__ __device__ constexpr int res_th(int KR) { return kResWarps * KR; }
@@ -49,8 +49,9 @@ __host__ __device__ constexpr unsigned res_smem(int KR) {
   return 8u * (kResSums * kResThreads + 3u * res_arr(KR)) + 16u * res_inbox(KR);
 }
 
-// The system of one solve.  Cell (i, j) at off + j * pitch + i of every array;
-// nothing outside 0 <= i < nx, 0 <= j < ny is read.
+// The system of one solve.  Cell (i, j) at off + j * pitch + i of every array; nothing
+// outside 0 <= i < nx, 0 <= j < ny is read, but for a mixed solve, whose residual reads
+// the ghost ring of a domain's padded layout (res_residual_padded).
 struct ResSys {
   int nx, ny;
   long pitch, off;

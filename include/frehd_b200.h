@@ -412,17 +412,19 @@ int frehd_cg_solve_noalloc(int nx, int ny, const double *Ct, const double *Gx, c
  * with the calls above, then admitted; while admitted, the batch steps it and
  * the single-domain step/state calls refuse it (FREHD_ERR_STATE).  Every
  * frehd_batch_step advances every admitted domain by one step with five kernel
- * launches in total (replayed from a CUDA graph where the driver accepts the
- * capture).  A domain's results do not depend on which other domains share the
- * batch.  The solve of all domains is one cooperative launch in one of two
- * packings (frehd_batch_set_cg_packing):
+ * launches in total, six in a batch whose solves run on chip and streamed, seven
+ * with both scalar advections besides (replayed from a CUDA graph where the driver
+ * accepts the capture).  A domain's results do not depend on which other domains
+ * share the batch.  The solves are cooperative launches in one of two packings
+ * (frehd_batch_set_cg_packing):
  *   FREHD_BATCH_CTA_GROUPS (default): a domain's CG runs on
  *     ceil(cells / cells_per_cta) CTAs (at most its tile count) whatever the mix; the
  *     single-CTA solves, largest first, go to whichever CTA is free; admission
  *     also needs free CTAs.  A domain whose solver state fits on chip (up to about
- *     600 K cells) runs instead on one CTA per tile of cells_per_cta cells (1024 to
- *     4096), the CTAs taking such solves one after another; its admission counts
- *     the same CTAs as before;
+ *     600 K cells; frehd_batch_set_resident) runs instead on one CTA per tile of
+ *     cells_per_cta cells (1024 to 4096), the CTAs taking such solves one after
+ *     another in a launch before the streaming one; admission counts the CTAs of
+ *     its group all the same;
  *   FREHD_BATCH_TILE_LIST: every domain's CG tiles form one list spread over
  *     all CTAs; a domain's sums are added in its own tile order, so its result is
  *     the same in any mix; cells_per_cta is not used, and admission is by memory
@@ -433,7 +435,7 @@ int frehd_cg_solve_noalloc(int nx, int ny, const double *Ct, const double *Gx, c
 typedef struct frehd_batch frehd_batch;
 typedef struct frehd_batch_info_t {
   int domains;             /* admitted domains */
-  int cg_ctas;             /* CTAs of the batched CG launch */
+  int cg_ctas;             /* CTAs of the batched CG launch (of the larger, if there are two) */
   int cg_capacity;         /* CTAs the device holds at once for it */
   long tiles;              /* blocks of each stencil kernel per step over all domains (each
                               runs up to four 32 x 8 tiles of one domain) */
