@@ -34,15 +34,24 @@ __device__ __forceinline__ void sys_of(const View &w, int x0_surface, int elimin
 // its solve starts, and its waits count, once all nb CTAs are there.  That wait ends too:
 // it gives up when no solve of the launch has shown a sign of life (a solve that ends,
 // or kResBeat reductions) for several times the longest that a solve waits in vain.
-__device__ __forceinline__ bool res_arrive(Scratch *sc, unsigned nb, unsigned *beat) {
-  atomicAdd(&sc->res_arrived, 1u);
+// (The caller has counted itself in.)
+__device__ __forceinline__ bool res_all_here(Scratch *sc, unsigned nb, unsigned *beat) {
+  volatile unsigned *arrived = &sc->res_arrived;
+  volatile int *status = &sc->status;
+  for (int n = 0; n < 64; ++n) {  // (both on their way together, and nothing else)
+    const unsigned here = *arrived;
+    const int st = *status;
+    if (st != FREHD_OK) return false;
+    if (here >= nb) return true;
+  }
   const unsigned long long own = sc->wait_limit_ns;
   const unsigned long long lim = 5 * (own > kBarrierTimeoutNs ? own : kBarrierTimeoutNs);
   unsigned seen = *(volatile unsigned *)beat;
   unsigned long long t0 = gtimer_ns();
-  while (*(volatile unsigned *)&sc->res_arrived < nb) {
-    if (*(volatile int *)&sc->status != FREHD_OK) return false;
-    const unsigned now = *(volatile unsigned *)beat;
+  for (;;) {
+    const unsigned here = *arrived, now = *(volatile unsigned *)beat;
+    if (*status != FREHD_OK) return false;
+    if (here >= nb) return true;
     if (now != seen) {
       seen = now;
       t0 = gtimer_ns();
@@ -51,7 +60,6 @@ __device__ __forceinline__ bool res_arrive(Scratch *sc, unsigned nb, unsigned *b
       return false;
     }
   }
-  return *(volatile int *)&sc->status == FREHD_OK;
 }
 
 // The two solves as functions of their own: in one kernel with each other or with
@@ -173,12 +181,14 @@ __global__ void __launch_bounds__(kResThreads, 1)
     __syncthreads();  // the previous job is done with the shared system
     if (threadIdx.x == 0) {
       const View *v = views2 + 2 * jb.d;
-      v += *(volatile int *)&v->sc->cur;
+      Scratch *sc = v->sc;
+      atomicAdd(&sc->res_arrived, 1u);
+      v += *(volatile int *)&sc->cur;
       sys_of(*v, jb.flags & 1, (jb.flags >> 1) & 1, &s_sys);
       s_sys.beat = &bsync->beat;
       s_mixed = v->p.mixed;
       s_eps = v->p.eps_inner;
-      s_run = res_arrive(v->sc, jb.nb, &bsync->beat);
+      s_run = res_all_here(sc, jb.nb, &bsync->beat);
     }
     __syncthreads();
     if (!s_run) continue;
