@@ -173,3 +173,53 @@ def test_a_start_that_meets_the_tolerance_is_returned(nx, ny):
     again, its, rel = _solve(system, eps=1e-6, x0=x)
     assert its == 0 and rel < 1e-6
     assert np.array_equal(again, x)
+
+
+@pytest.mark.parametrize("nx,ny", [(48, 40), (130, 500), (512, 512), (24, 10922)])
+def test_queued_solve_captured_in_a_graph(nx, ny):
+    """The solve queued on a capturing stream (after a first call, which sets the device
+    up) and replayed on new right-hand sides: the direct call's doubles."""
+    import torch
+    system = _signed_system(nx, ny)
+    bufs = [torch.from_numpy(a.ravel().copy()).cuda() for a in system]
+    x = torch.zeros(nx * ny, dtype=torch.float64, device="cuda")
+    _solve(system)
+    s, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        native.cg_solve_noalloc(nx, ny, *[t.data_ptr() for t in bufs], x.data_ptr(), 1e-12, 1000,
+                                stream=torch.cuda.current_stream().cuda_stream, wait=False)
+    for k in range(3):
+        b = np.random.default_rng(k).standard_normal((ny, nx))
+        bufs[3].copy_(torch.from_numpy(b.ravel()))
+        g.replay()
+        torch.cuda.synchronize()
+        want, _, _ = _solve([*system[:3], b])
+        assert np.array_equal(x.cpu().numpy().reshape(ny, nx), want)
+
+
+def test_domains_of_several_host_threads():
+    """Solves of 16, 64 and 128 CTAs in and out of clusters on streams of their own, which
+    do not all fit the device at once: the doubles of each domain stepped alone."""
+    import threading
+
+    from frehdc_b200 import deck as D
+    sizes = [(128, 128), (256, 256), (512, 512), (500, 520), (70, 40), (130, 500)]
+    decks = [D.make_deck(D.DeckSpec(nx=nx, ny=ny, steps=60, seed=25 + k, dry_frac=0.2))
+             for k, (nx, ny) in enumerate(sizes)]
+    precs = [native.PRECISION_MIXED if k % 2 else native.PRECISION_FP64 for k in range(len(decks))]
+    doms = [native.domain_from_deck(d, precision=p) for d, p in zip(decks, precs)]
+    status = [None] * len(doms)
+
+    def steps(k):
+        status[k] = [doms[k].run(1 + 10 * n, 10) for n in range(5)]
+    threads = [threading.Thread(target=steps, args=(k,)) for k in range(len(doms))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k, (g, d) in enumerate(zip(doms, decks)):
+        assert status[k] == [0] * 5
+        alone = native.domain_from_deck(d, precision=precs[k])
+        assert alone.run(1, 50) == 0
+        for f in ("surf", "uuXP", "vvYP", "S"):
+            assert np.array_equal(g.download([f])[f], alone.download([f])[f]), (k, f)
