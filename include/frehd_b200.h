@@ -381,7 +381,11 @@ int frehd_domain_set_precision(frehd_domain *d, int mode, double eps_inner);
  * couplings), Gx[k] the coupling across the east face of cell k, Gy[k] across
  * its north face (0 on the domain edge), b the right-hand side.  Solves to
  * ||r||_2 < eps*||b||_2 or max_iter iterations with the same Jacobi-PCG as
- * the domain step.  x0_from_x = 0 starts from x = 0, else from the x passed in.
+ * the domain step, r being the recurrence's residual of the system scaled by
+ * sqrt|Ct|: past about 1000 iterations an eps near the rounding level of the
+ * system is met by r, while x is as good as the condition number allows.
+ * x0_from_x = 0 starts from x = 0, else from the x passed in, which is returned
+ * as it was if it meets eps already.
  *
  * Limit: nx*ny <= 512*512 cells; larger sizes return FREHD_ERR_INVALID.  The
  * solve's work vectors live in a static device array inside the library
